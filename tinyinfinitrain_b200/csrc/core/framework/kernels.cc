@@ -3,7 +3,7 @@
 //
 // CPU tensors: ATen fp32 math restating infini_train/src/kernels/cpu/*.cc (the numerical oracle).
 // CUDA float32/bfloat16 tensors: the sm_100a kernel library (tcgen05 GEMM for bf16 Linear/Matmul,
-// the SIMT SGEMM for fp32, fused LayerNorm / softmax / cross-entropy / embedding / Adam kernels);
+// the split-bf16 SGEMM for fp32, fused LayerNorm / softmax / cross-entropy / embedding / Adam kernels);
 // reductions, outer product, mask, tril/triu and every materialised view (transpose, slice, split, stack,
 // repeat-interleave) go through the library's reduce / gather / scatter kernels as well.
 #include <ATen/cuda/CUDAContext.h>

@@ -101,7 +101,7 @@ TITB_API int titb_gemm_pick_tile(int M, int N, int K, int splits);
 TITB_API int titb_gemm_split_in_place(const TitbGemmDesc* d);
 // Switches the shared-memory-staged TMA store epilogue of bf16 outputs on (default) or off (A/B timing).
 TITB_API void titb_gemm_set_tma_store(int enabled);
-// fp32 SIMT GEMM for API parity with fp32 tensors: C[M,N] (+)= op(A) op(B), row-major.
+// fp32 GEMM at fp32 accuracy (sgemm.cu): C[M,N] (+)= op(A) op(B), row-major.
 TITB_API int titb_sgemm(const float* A, const float* B, float* C, int M, int N, int K, int trans_a, int trans_b,
                         int accumulate, cudaStream_t stream);
 

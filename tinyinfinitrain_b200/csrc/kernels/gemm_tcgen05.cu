@@ -1555,62 +1555,3 @@ TITB_API int TITB_GEMM_ENTRY(const TitbGemmDesc* d, cudaStream_t stream) {
   }
   return rc;
 }
-
-#ifndef TITB_GEMM_PARAM_GATHER
-// ------------------------------------------------------------- fp32 SIMT GEMM
-// Kept for fp32 tensors on the GPU (API parity with the reference's fp32-only
-// Matmul/Linear); not a hot path.  64x64 tile, 16-deep k slab, 4x4 per thread.
-namespace titb {
-__global__ void __launch_bounds__(256) sgemm_kernel(const float* __restrict__ A, const float* __restrict__ B,
-                                                    float* __restrict__ C, int M, int N, int K, int ta, int tb,
-                                                    int accumulate) {
-  __shared__ float As[16][64 + 1];
-  __shared__ float Bs[16][64 + 1];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < K; k0 += 16) {
-    for (int i = threadIdx.x; i < 64 * 16; i += 256) {
-      int kk = i & 15, mm = i >> 4;
-      int gm = m0 + mm, gk = k0 + kk;
-      float va = 0.f, vb = 0.f;
-      if (gm < M && gk < K) va = ta ? A[(long long)gk * M + gm] : A[(long long)gm * K + gk];
-      int gn = n0 + mm;
-      if (gn < N && gk < K) vb = tb ? B[(long long)gn * K + gk] : B[(long long)gk * N + gn];
-      As[kk][mm] = va;
-      Bs[kk][mm] = vb;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < 16; ++kk) {
-      float a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-  for (int i = 0; i < 4; ++i)
-    for (int j = 0; j < 4; ++j) {
-      int gm = m0 + ty * 4 + i, gn = n0 + tx * 4 + j;
-      if (gm < M && gn < N) {
-        float* c = C + (long long)gm * N + gn;
-        *c = accumulate ? *c + acc[i][j] : acc[i][j];
-      }
-    }
-}
-}  // namespace titb
-
-TITB_API int titb_sgemm(const float* A, const float* B, float* C, int M, int N, int K, int trans_a, int trans_b,
-                        int accumulate, cudaStream_t stream) {
-  if (M <= 0 || N <= 0) return 0;
-  dim3 grid((N + 63) / 64, (M + 63) / 64);
-  titb::sgemm_kernel<<<grid, 256, 0, stream>>>(A, B, C, M, N, K, trans_a, trans_b, accumulate);
-  return static_cast<int>(cudaGetLastError());
-}
-#endif  // !TITB_GEMM_PARAM_GATHER

@@ -1,8 +1,8 @@
 """Autograd functions over the sm_100a kernels, with CPU reference paths.
 
 Each public function takes torch tensors.  CUDA tensors run the hand-written
-kernels of ``csrc/kernels`` (bf16 on tcgen05 tensor cores, fp32 on SIMT
-kernels for API parity); CPU tensors run plain PyTorch fp32 math, which is the
+kernels of ``csrc/kernels`` (bf16 on tcgen05 tensor cores, fp32 GEMMs there
+too, as exact three-way bf16 splits); CPU tensors run plain PyTorch fp32 math, which is the
 numerical oracle the GPU tests compare against.
 
 Weight gradients: a parameter that carries a ``main_grad`` attribute (an fp32
@@ -117,7 +117,7 @@ class _LinearFn(torch.autograd.Function):
 
 
 class _LinearF32Fn(torch.autograd.Function):
-    """fp32 tensors on the GPU: SIMT SGEMM (API parity with the reference's fp32 Linear)."""
+    """fp32 tensors on the GPU: the split-bf16 tensor-core GEMM at fp32 accuracy (csrc/kernels/sgemm.cu)."""
 
     @staticmethod
     def forward(ctx, x, w, b):
