@@ -118,7 +118,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
   const int nqb = (p.T + kBlk - 1) / kBlk;
   const int qb = nqb - 1 - blockIdx.x;  // heaviest tiles first
   const int h = blockIdx.y, b = blockIdx.z;
@@ -156,7 +156,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
   if (bad_align) {
     // fall through to the common exit
   } else if (warp == 0) {
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       ptx::mbar_expect_tx(q_full, Cfg::kTileBytes);
 #pragma unroll
       for (int c = 0; c < HD / 64; ++c)
@@ -178,7 +178,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       const uint32_t idesc_s = ptx::make_idesc_bf16(128, 128, 0, 0);
       const uint32_t idesc_o = ptx::make_idesc_bf16(128, HD, 0, 1);
       const uint32_t q_base = ptx::smem_u32(smem + Cfg::kQ);
@@ -419,7 +419,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
   const int nqb = (p.T + kBlk - 1) / kBlk;
   const int jb = blockIdx.x;  // key block
   const int hk = blockIdx.y, b = blockIdx.z;
@@ -454,7 +454,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
 
   if (bad_align) {
   } else if (warp == 0) {
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       ptx::mbar_expect_tx(kv_full, 2 * Cfg::kTileBytes);
 #pragma unroll
       for (int c = 0; c < HD / 64; ++c) {
@@ -477,7 +477,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       const uint32_t idesc_s = ptx::make_idesc_bf16(128, 128, 0, 0);   // S, dP : K-major x K-major
       const uint32_t idesc_t = ptx::make_idesc_bf16(128, HD, 1, 1);    // dV, dK: MN-major x MN-major
       const uint32_t idesc_q = ptx::make_idesc_bf16(128, HD, 0, 1);    // dQ    : K-major x MN-major

@@ -594,7 +594,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(aux_bar + 1);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = ptx::warp_index();
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -635,7 +635,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -727,7 +727,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------- MMA issuer
-    if (lane == 0 && pair_rank == 0) {
+    if (pair_rank == 0 && ptx::elect_one()) {
       const uint32_t idesc = ptx::make_idesc_bf16(kTileM, BN, p.a_mn, p.b_mn);
       int stage = 0;
       uint32_t phase = 0;

@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(kSThreads, 1) sgemm_split3_kernel(const SgemmA
   uint64_t* acc_empty = acc_full + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile uint32_t* abort_flag = tmem_slot + 1;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kSStages; ++s) {
@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(kSThreads, 1) sgemm_split3_kernel(const SgemmA
     }
   } else if (warp == kConvWarps + kDrainWarps) {
     // ------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       const uint32_t idesc = ptx::make_idesc_bf16(kST, kST, p.a_mn, p.b_mn);
       const uint32_t a_lbo = p.a_mn ? 64 * kSK * 2 : 16, b_lbo = p.b_mn ? 64 * kSK * 2 : 16;
       const uint32_t a_step = p.a_mn ? 16 * 128 : 32, b_step = p.b_mn ? 16 * 128 : 32;
