@@ -26,6 +26,28 @@ def _status_ok():
 
 
 
+@pytest.mark.parametrize("B,T,Hq,Hkv,hd", [(3, 1, 2, 2, 64), (2, 127, 2, 1, 128), (2, 129, 4, 2, 128), (3, 257, 2, 1, 64)])
+def test_attention_backward_tiles_end_with_their_sequence(B, T, Hq, Hkv, hd):
+    """The last tile of a sequence reads zeros past its end and adds nothing there: NaNs in the other sequences leave the
+    gradients of sequence 0 as they were (dK and dV to the bit; dQ is a sum of at most three partials in any order, each
+    addition rounding to 2^-24, before it is rounded to bf16: one bf16 step of the largest value)."""
+    torch.manual_seed(23)
+    q = torch.randn(B, T, Hq, hd, device=DEV).to(BF)
+    k, v = (torch.randn(B, T, Hkv, hd, device=DEV).to(BF) for _ in range(2))
+    do = torch.randn(B, T, Hq, hd, device=DEV).to(BF)
+    scale = hd ** -0.5
+    o, lse = C.attn_fwd(q, k, v, scale)
+    clean = [g.clone() for g in C.attn_bwd(do, q, k, v, o, lse, scale)]
+    for t in (q, k, v, do):
+        t[1:] = float("nan")
+    poisoned = C.attn_bwd(do, q, k, v, o, lse, scale)
+    torch.cuda.synchronize()
+    _status_ok()
+    assert torch.equal(poisoned[1][0], clean[1][0]) and torch.equal(poisoned[2][0], clean[2][0])
+    bound = clean[0][0].abs().max().item() * 2.0 ** -7
+    assert (poisoned[0][0].float() - clean[0][0].float()).abs().max().item() <= bound   # also false for NaN
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, BF])
 @pytest.mark.parametrize("rows,cols", [(8192, 768), (1000, 1024), (4737, 512), (37, 256), (5, 64), (300, 2048), (64, 4096)])
 @pytest.mark.parametrize("rms", [False, True])

@@ -15,11 +15,11 @@
 //
 //   backward, one CTA per (128 key rows, kv head, batch), loop over query blocks i >= j
 //   and over the query heads that share the kv head (GQA):
-//     S = Q_i K_j^T, dP = dO_i V_j^T            -> TMEM
-//     P = exp(S - lse), dS = P (dP - delta)     -> smem (bf16), both stored once and read
-//                                                  as K-major and as MN-major operands
+//     S^T = K_j Q_i^T, dP^T = V_j dO_i^T        -> TMEM
+//     P = exp(S - lse), dS = P (dP - delta)     -> P^T (bf16) in TMEM, dS^T (bf16) in smem, read as
+//                                                  a K-major and as an MN-major operand
 //     dV += P^T dO_i, dK += dS^T Q_i            accumulate in TMEM over the whole loop
-//     dQ_i += dS K_j                            TMEM -> fp32 vector reductions in HBM
+//     dQ_i += dS K_j                            TMEM -> smem -> fp32 TMA reduce-adds in HBM
 //
 // q/k/v are addressed in place inside a fused projection buffer through TMA tensor
 // maps (row stride = token stride), so no split/transpose kernel runs.  All waits
@@ -36,8 +36,8 @@ namespace titb {
 
 bool make_tmap_bf16_2d(CUtensorMap* m, const void* base, uint64_t inner, uint64_t outer, uint64_t ld,
                        uint32_t box_inner, uint32_t box_outer);
-bool make_tmap_f32_2d(CUtensorMap* m, const void* base, uint64_t inner, uint64_t outer, uint64_t ld,
-                      uint32_t box_inner, uint32_t box_outer);
+bool make_tmap_tokens(CUtensorMap* m, const void* base, int fp32, uint64_t width, uint64_t T, uint64_t B, uint64_t ld,
+                      uint32_t box_width, uint32_t box_tokens);
 
 constexpr int kAttnThreads = 192;
 constexpr int kBlk = 128;             // query rows per CTA tile and keys per step
@@ -359,90 +359,125 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
 }
 
 // ------------------------------------------------------------------------ backward
+// Warps 0..7 element-wise, 8..11 dQ, 12 loads, 13 MMA issue.
+constexpr int kBwdThreads = 448;
+
 template <int HD>
 struct BwdCfg {
   static constexpr int kTileBytes = kBlk * HD * 2;
-  // Q / dO tiles of the coming iterations: with three stages a load is issued a whole iteration before its tile is
-  // needed (two stages left no lead at all: the slot of iteration it+1 is only released by iteration it-1)
-  static constexpr int kStages = (HD == 64) ? 3 : 1;
-  static constexpr bool kAliasDq = (HD > 64);  // dQ partial reuses the S columns when TMEM is full
+  static constexpr bool kAlias = (HD == 128);       // tensor memory is full: P lies over S, dQ over dP
+  static constexpr int kDoStages = (HD == 64) ? 2 : 1;
   static constexpr int kK = 0;
   static constexpr int kV = kK + kTileBytes;
-  static constexpr int kQ = kV + kTileBytes;
-  static constexpr int kDO = kQ + kStages * kTileBytes;
-  static constexpr int kP = kDO + kStages * kTileBytes;
-  static constexpr int kDS = kP + kBlk * kBlk * 2;
-  // hd 64: two [128 rows x 32 fp32] staging tiles from which dQ leaves by TMA reduce-add (hd 128 has no room and
-  // flushes dQ with vector reductions from registers)
-  static constexpr int kDQ = kDS + kBlk * kBlk * 2;
-  static constexpr int kDQBytes = kAliasDq ? 0 : 2 * kBlk * 128;
-  static constexpr int kBar = kDQ + kDQBytes;
-  static constexpr int kSmem = kBar + 128;
+  static constexpr int kQ = kV + kTileBytes;        // two stages
+  static constexpr int kDO = kQ + 2 * kTileBytes;
+  static constexpr int kDS = kDO + kDoStages * kTileBytes;
+  static constexpr int kDQ = kDS + kBlk * kBlk * 2; // per dQ warp two [32 rows x 32 fp32] tiles that leave by TMA
+  static constexpr int kStat = kDQ + 4 * 2 * 4096;  // per Q stage: 128 x (-lse log2 e), 128 x delta
+  static constexpr int kBar = kStat + 2 * 2 * kBlk * 4;
+  static constexpr int kSmem = kBar + 256;
   static constexpr int kTmemCols = 512;
   static constexpr int kColS = 0, kColDP = 128, kColDV = 256, kColDK = 256 + HD;
-  static constexpr int kColDQ = kAliasDq ? 0 : 256 + 2 * HD;
+  static constexpr int kColDQ = kAlias ? kColDP : 384;
+  // bf16 P, two queries per column: query half h starts at kColP + h * kPHalf
+  static constexpr int kColP = kAlias ? kColS : 448;
+  static constexpr int kPHalf = kAlias ? 64 : 32;
 };
 
-__device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+// two fp32 operations per instruction
+__device__ __forceinline__ void fma2(float& a0, float& a1, float b0, float b1, float c0, float c1, float d0, float d1) {
+  asm("{\n\t.reg .b64 x, y, z;\n\t"
+      "mov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+      "fma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(a0), "=f"(a1) : "f"(b0), "f"(b1), "f"(c0), "f"(c1), "f"(d0), "f"(d1));
+}
+__device__ __forceinline__ void mul2(float& a0, float& a1, float b0, float b1, float c0, float c1) {
+  asm("{\n\t.reg .b64 x, y;\n\t"
+      "mov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+      "mul.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(a0), "=f"(a1) : "f"(b0), "f"(b1), "f"(c0), "f"(c1));
+}
+__device__ __forceinline__ void add2(float& a0, float& a1, float b0, float b1, float c0, float c1) {
+  asm("{\n\t.reg .b64 x, y;\n\t"
+      "mov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+      "add.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(a0), "=f"(a1) : "f"(b0), "f"(b1), "f"(c0), "f"(c1));
 }
 
-// Backward pipeline.  Warps 2..9 are the element-wise warps: a score row is shared by two warps (warps 2..5 take
-// key columns 0..63 and the first half of the head dimension, warps 6..9 the second halves; both sets sit on the
-// TMEM lane quarter `warp & 3`).  Per (query head, query block) iteration `it`:
-//   MMA warp:  S(it+1), dP(it+1) are issued as soon as the element-wise warps have copied S(it), dP(it) out of
-//              tensor memory (sdp_free), so they run underneath the exponentials of iteration it; dV, dK
-//              accumulate over the whole loop; dQ(it) is issued when the element-wise warps have flushed dQ(it-1).
-//   EW warps:  S and dP of their 64 columns are read from tensor memory once (128 registers), P and dS are
-//              computed from registers, stored to shared memory once MMA group 2 of iteration it-1 has finished
-//              reading the buffers, and only then is dQ(it-1) flushed to HBM -- underneath dV(it), dK(it).
-// With hd = 128 tensor memory is full and dQ shares the S columns, so S(it+1) has to wait for the dQ(it) flush:
-// that instantiation keeps the order S, dP -> P, dS -> dV, dK, dQ -> flush.
+// Backward pipeline.  Scores are computed transposed (rows = keys, columns = queries), so that P^T can stay in tensor
+// memory as the A operand of dV and only dS passes through shared memory, stored once and read as the K-major A operand
+// of dK and as the MN-major A operand of dQ.  Per (query head, query block) iteration `it` the MMA warp issues
+//     dV += P^T dO (it) | S^T = K Q^T (it+1) | dQ = dS K (it) | dK += dS^T Q (it) | dP^T = V dO^T (it+1)
+// and the other warps work beside it:
+//   element-wise warps: exponentials of it+1 under dQ, dK (it); dS of it+1 under dV (it+1), S (it+2).  Two warps share a
+//     key row (query columns 0..63 and 64..127).  The row statistics of the queries are columns here; they come from
+//     shared memory as broadcast reads.
+//   dQ warps: copy dQ(it) out of tensor memory and add it to the fp32 accumulator by TMA reduce-adds of 32 x 32 tiles,
+//     each warp on its own.
+// MMAs execute in issue order, which orders most reuses: S(it+1) overwrites P(it) (hd 128) after dV(it) has read it, and
+// dp_full(it+1) tells that dQ(it), dK(it) have read the dS buffer.
+// Bound: at hd 128 the five products read 5 x 512 cycles of shared-memory operands an iteration, and dS, dQ and the loads
+// move as much again; at hd 64 the 16384 exponentials take 1024 cycles and the products 1660.
+// Measured (B200, with the delta and conversion passes; before = scores untransposed, P and dS through shared memory, dQ
+// flushed by the element-wise warps): hd 128, 1 x 4096, 32 / 8 heads: 978 -> 351 us (980 TFLOP/s); hd 64, 4 x 2048,
+// 32 / 8 heads: 376 -> 249 us; 8 x 1024, 12 heads: 117 -> 91 us; 3 x 777, 12 heads: 50 -> 32 us.
 template <int HD>
-__global__ void __launch_bounds__(320, 1)
+__global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                 const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
                 const __grid_constant__ CUtensorMap tdq, const AttnArgs p) {
   using Cfg = BwdCfg<HD>;
-  constexpr int S = Cfg::kStages;
-  constexpr bool kPipe = !Cfg::kAliasDq;
+  constexpr int DS = Cfg::kDoStages;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::kBar);
   uint64_t* kv_full = bars;            // 1
-  uint64_t* qdo_full = bars + 1;       // [3]
-  uint64_t* qdo_empty = bars + 4;      // [3]
-  uint64_t* sdp_full = bars + 7;
-  uint64_t* pds_full = bars + 8;
-  uint64_t* dq_full = bars + 9;
-  uint64_t* dq_free = bars + 10;
-  uint64_t* sdp_free = bars + 11;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
+  uint64_t* q_full = bars + 1;         // [2]
+  uint64_t* q_empty = bars + 3;        // [2]
+  uint64_t* do_full = bars + 5;        // [2]
+  uint64_t* do_empty = bars + 7;       // [2]
+  uint64_t* stat_full = bars + 9;      // [2]  freed with the Q stage
+  uint64_t* s_full = bars + 11;
+  uint64_t* p_full = bars + 12;
+  uint64_t* dp_full = bars + 13;
+  uint64_t* ds_full = bars + 14;
+  uint64_t* dq_full = bars + 15;
+  uint64_t* dq_free = bars + 16;
+  uint64_t* dkv_full = bars + 17;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
   const int nqb = (p.T + kBlk - 1) / kBlk;
-  const int jb = blockIdx.x;  // key block
-  const int hk = blockIdx.y, b = blockIdx.z;
+  // key block 0 meets every query block: the longest CTAs of all heads start first
+  const int jb = blockIdx.y;
+  const int hk = blockIdx.x % p.Hkv, b = blockIdx.x / p.Hkv;
   const int G = p.Hq / p.Hkv;
   const int nq = nqb - jb;     // query blocks jb .. nqb-1
   const int niter = G * nq;
 
   if (threadIdx.x == 0) {
     ptx::mbar_init(kv_full, 1);
-    for (int s = 0; s < 3; ++s) { ptx::mbar_init(&qdo_full[s], 1); ptx::mbar_init(&qdo_empty[s], 1); }
-    ptx::mbar_init(sdp_full, 1);
-    ptx::mbar_init(pds_full, 8);
+    for (int s = 0; s < 2; ++s) {
+      ptx::mbar_init(&q_full[s], 1); ptx::mbar_init(&q_empty[s], 1);
+      ptx::mbar_init(&do_full[s], 1); ptx::mbar_init(&do_empty[s], 1);
+      ptx::mbar_init(&stat_full[s], 1);
+    }
+    ptx::mbar_init(s_full, 1);
+    ptx::mbar_init(p_full, 8);
+    ptx::mbar_init(dp_full, 1);
+    ptx::mbar_init(ds_full, 8);
     ptx::mbar_init(dq_full, 1);
-    ptx::mbar_init(dq_free, 8);
-    ptx::mbar_init(sdp_free, 8);
+    ptx::mbar_init(dq_free, 4);
+    ptx::mbar_init(dkv_full, 1);
     *abort_flag = (ptx::smem_u32(smem) & 1023u) ? 1u : 0u;
     ptx::mbar_fence_init();
     ptx::tma_prefetch_desc(&tq);
     ptx::tma_prefetch_desc(&tk);
     ptx::tma_prefetch_desc(&tv);
     ptx::tma_prefetch_desc(&tdo);
+    ptx::tma_prefetch_desc(&tdq);
   }
-  if (warp == 1) {
+  if (warp == 13) {
     ptx::tmem_alloc(tmem_slot, Cfg::kTmemCols);
     ptx::tmem_relinquish();
   }
@@ -453,258 +488,284 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
   const bool bad_align = (*abort_flag != 0);
 
   if (bad_align) {
-  } else if (warp == 0) {
-    if (ptx::elect_one()) {
+    // fall through to the common exit
+  } else if (warp == 12) {
+    // ------------------------------------------------------------ loads
+    const bool leader = ptx::elect_one();
+    if (leader) {
       ptx::mbar_expect_tx(kv_full, 2 * Cfg::kTileBytes);
 #pragma unroll
       for (int c = 0; c < HD / 64; ++c) {
-        ptx::tma_load_2d(smem + Cfg::kK + c * kChunkBytes, &tk, kv_full, hk * HD + c * 64, b * p.T + jb * kBlk);
-        ptx::tma_load_2d(smem + Cfg::kV + c * kChunkBytes, &tv, kv_full, hk * HD + c * 64, b * p.T + jb * kBlk);
+        ptx::tma_load_3d(smem + Cfg::kK + c * kChunkBytes, &tk, kv_full, hk * HD + c * 64, jb * kBlk, b);
+        ptx::tma_load_3d(smem + Cfg::kV + c * kChunkBytes, &tv, kv_full, hk * HD + c * 64, jb * kBlk, b);
       }
-      for (int it = 0; it < niter; ++it) {
-        const int g = it / nq, i = jb + (it - g * nq);
-        const int h = hk * G + g;
-        const int st = it % S;
-        if (!ptx::mbar_wait(&qdo_empty[st], ((it / S) & 1) ^ 1u, abort_flag)) break;
-        ptx::mbar_expect_tx(&qdo_full[st], 2 * Cfg::kTileBytes);
+    }
+    bool ok = true;
+    int it = 0;
+    for (; it < niter; ++it) {
+      const int g = it / nq, i = jb + (it - g * nq);
+      const int h = hk * G + g;
+      const int st = it & 1, dst = it % DS;
+      // row statistics: requested before the waits; rows past the end of the sequence get lse = +inf, which turns their
+      // probabilities into exact zeros
+      float l[4], d[4];
+      const float* lse_row = p.lse + (static_cast<long long>(b) * p.Hq + h) * p.T;
+      const float* dlt_row = p.delta + (static_cast<long long>(b) * p.Hq + h) * p.T;
 #pragma unroll
-        for (int c = 0; c < HD / 64; ++c) {
-          ptx::tma_load_2d(smem + Cfg::kQ + st * Cfg::kTileBytes + c * kChunkBytes, &tq, &qdo_full[st],
-                           h * HD + c * 64, b * p.T + i * kBlk);
-          ptx::tma_load_2d(smem + Cfg::kDO + st * Cfg::kTileBytes + c * kChunkBytes, &tdo, &qdo_full[st],
-                           h * HD + c * 64, b * p.T + i * kBlk);
+      for (int e = 0; e < 4; ++e) {
+        const int q = i * kBlk + e * 32 + lane;
+        l[e] = q < p.T ? lse_row[q] : INFINITY;
+        d[e] = q < p.T ? dlt_row[q] : 0.f;
+      }
+      ok = ptx::mbar_wait(&q_empty[st], ((it >> 1) & 1) ^ 1u, abort_flag);
+      if (__any_sync(0xffffffffu, !ok)) break;
+      if (leader) {
+        ptx::mbar_expect_tx(&q_full[st], Cfg::kTileBytes);
+#pragma unroll
+        for (int c = 0; c < HD / 64; ++c)
+          ptx::tma_load_3d(smem + Cfg::kQ + st * Cfg::kTileBytes + c * kChunkBytes, &tq, &q_full[st], h * HD + c * 64,
+                           i * kBlk, b);
+      }
+      float* stat = reinterpret_cast<float*>(smem + Cfg::kStat) + st * 2 * kBlk;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        stat[e * 32 + lane] = -l[e] * kLog2e;
+        stat[kBlk + e * 32 + lane] = d[e];
+      }
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(&stat_full[st]);
+      ok = ptx::mbar_wait(&do_empty[dst], ((it / DS) & 1) ^ 1u, abort_flag);
+      if (__any_sync(0xffffffffu, !ok)) break;
+      if (leader) {
+        ptx::mbar_expect_tx(&do_full[dst], Cfg::kTileBytes);
+#pragma unroll
+        for (int c = 0; c < HD / 64; ++c)
+          ptx::tma_load_3d(smem + Cfg::kDO + dst * Cfg::kTileBytes + c * kChunkBytes, &tdo, &do_full[dst], h * HD + c * 64,
+                           i * kBlk, b);
+      }
+    }
+    if (it < niter && leader) {
+      // gave up: copies already issued get a bounded chance to land before the CTA leaves
+      const long long t0 = clock64();
+      for (int s = 0; s < 5; ++s) {
+        uint64_t* bar = s < 2 ? &q_full[s] : s < 4 ? &do_full[s - 2] : kv_full;
+        while (!ptx::mbar_try_wait(bar, 0) && !ptx::mbar_try_wait(bar, 1) && clock64() - t0 < 4000000LL) {
         }
       }
     }
-  } else if (warp == 1) {
+  } else if (warp == 13) {
+    // ------------------------------------------------------------ MMA issue
     if (ptx::elect_one()) {
-      const uint32_t idesc_s = ptx::make_idesc_bf16(128, 128, 0, 0);   // S, dP : K-major x K-major
-      const uint32_t idesc_t = ptx::make_idesc_bf16(128, HD, 1, 1);    // dV, dK: MN-major x MN-major
-      const uint32_t idesc_q = ptx::make_idesc_bf16(128, HD, 0, 1);    // dQ    : K-major x MN-major
+      const uint32_t idesc_s = ptx::make_idesc_bf16(128, 128, 0, 0);    // S^T, dP^T: K-major x K-major
+      const uint32_t idesc_kv = ptx::make_idesc_bf16(128, HD, 0, 1);    // dV (A in tensor memory), dK: K-major x MN-major
+      const uint32_t idesc_q = ptx::make_idesc_bf16(128, HD, 1, 1);     // dQ: MN-major x MN-major
       const uint32_t k_base = ptx::smem_u32(smem + Cfg::kK), v_base = ptx::smem_u32(smem + Cfg::kV);
-      const uint32_t p_base = ptx::smem_u32(smem + Cfg::kP), ds_base = ptx::smem_u32(smem + Cfg::kDS);
-      // descriptors of the fixed tiles, and of stage 0 of the Q / dO ring, in both operand layouts
+      const uint32_t ds_base = ptx::smem_u32(smem + Cfg::kDS);
+      const uint32_t q_base0 = ptx::smem_u32(smem + Cfg::kQ), do_base0 = ptx::smem_u32(smem + Cfg::kDO);
       const uint64_t k_kmaj = ptx::make_smem_desc(k_base, 16, 1024), v_kmaj = ptx::make_smem_desc(v_base, 16, 1024);
       const uint64_t k_mn = ptx::make_smem_desc(k_base, kChunkBytes, 1024);
-      const uint64_t p_mn = ptx::make_smem_desc(p_base, kChunkBytes, 1024), ds_mn = ptx::make_smem_desc(ds_base, kChunkBytes, 1024);
-      const uint64_t ds_kmaj = ptx::make_smem_desc(ds_base, 16, 1024);
-      const uint32_t q_base0 = ptx::smem_u32(smem + Cfg::kQ), do_base0 = ptx::smem_u32(smem + Cfg::kDO);
+      const uint64_t ds_kmaj = ptx::make_smem_desc(ds_base, 16, 1024), ds_mn = ptx::make_smem_desc(ds_base, kChunkBytes, 1024);
       const uint64_t q_kmaj0 = ptx::make_smem_desc(q_base0, 16, 1024), do_kmaj0 = ptx::make_smem_desc(do_base0, 16, 1024);
       const uint64_t q_mn0 = ptx::make_smem_desc(q_base0, kChunkBytes, 1024), do_mn0 = ptx::make_smem_desc(do_base0, kChunkBytes, 1024);
-      auto issue_sdp = [&](int it) {
-        const uint32_t st_off = (it % S) * Cfg::kTileBytes;
-        const uint64_t q_d = desc_add(q_kmaj0, st_off), do_d = desc_add(do_kmaj0, st_off);
+      auto issue_s = [&](int it) {
+        const uint64_t q_d = desc_add(q_kmaj0, (it & 1) * Cfg::kTileBytes);
 #pragma unroll
         for (int k = 0; k < HD / 16; ++k) {
           const uint32_t off = (k >> 2) * kChunkBytes + (k & 3) * 32;
-          ptx::mma_f16_ss(tmem_base + Cfg::kColS, desc_add(q_d, off), desc_add(k_kmaj, off), idesc_s, k > 0);
+          ptx::mma_f16_ss(tmem_base + Cfg::kColS, desc_add(k_kmaj, off), desc_add(q_d, off), idesc_s, k > 0);
         }
-#pragma unroll
-        for (int k = 0; k < HD / 16; ++k) {
-          const uint32_t off = (k >> 2) * kChunkBytes + (k & 3) * 32;
-          ptx::mma_f16_ss(tmem_base + Cfg::kColDP, desc_add(do_d, off), desc_add(v_kmaj, off), idesc_s, k > 0);
-        }
-        ptx::tc_commit(sdp_full);
+        ptx::tc_commit(s_full);
       };
-      bool ok = ptx::mbar_wait(kv_full, 0, abort_flag);
-      if (ok && niter > 0) {
-        ok = ptx::mbar_wait(&qdo_full[0], 0, abort_flag);
-        if (ok) {
-          ptx::tc_fence_after_sync();
-          issue_sdp(0);
+      auto issue_dp = [&](int it) {
+        const uint64_t do_d = desc_add(do_kmaj0, (it % DS) * Cfg::kTileBytes);
+#pragma unroll
+        for (int k = 0; k < HD / 16; ++k) {
+          const uint32_t off = (k >> 2) * kChunkBytes + (k & 3) * 32;
+          ptx::mma_f16_ss(tmem_base + Cfg::kColDP, desc_add(v_kmaj, off), desc_add(do_d, off), idesc_s, k > 0);
         }
+        ptx::tc_commit(dp_full);
+      };
+      bool ok = ptx::mbar_wait(kv_full, 0, abort_flag) && ptx::mbar_wait(&q_full[0], 0, abort_flag);
+      if (ok) {
+        ptx::tc_fence_after_sync();
+        issue_s(0);
+        ok = ptx::mbar_wait(&do_full[0], 0, abort_flag);
+      }
+      if (ok) {
+        ptx::tc_fence_after_sync();
+        issue_dp(0);
       }
       for (int it = 0; it < niter && ok; ++it) {
-        const int st = it % S;
-        const uint64_t q_m = desc_add(q_mn0, st * Cfg::kTileBytes), do_m = desc_add(do_mn0, st * Cfg::kTileBytes);
-        if (kPipe && it + 1 < niter) {
-          // next S / dP: operands loaded, and the score columns copied out by the element-wise warps
-          if (!ptx::mbar_wait(&qdo_full[(it + 1) % S], ((it + 1) / S) & 1, abort_flag)) break;
-          if (!ptx::mbar_wait(sdp_free, it & 1, abort_flag)) break;
-          ptx::tc_fence_after_sync();
-          issue_sdp(it + 1);
-        }
-        if (!ptx::mbar_wait(pds_full, it & 1, abort_flag)) break;
+        const uint64_t q_m = desc_add(q_mn0, (it & 1) * Cfg::kTileBytes), do_m = desc_add(do_mn0, (it % DS) * Cfg::kTileBytes);
+        if (!ptx::mbar_wait(p_full, it & 1, abort_flag)) break;
         ptx::tc_fence_after_sync();
 #pragma unroll
-        for (int k = 0; k < kBlk / 16; ++k) {  // reduction over the 128 query rows
-          ptx::mma_f16_ss(tmem_base + Cfg::kColDV, desc_add(p_mn, k * 2048), desc_add(do_m, k * 2048), idesc_t, (it > 0 || k > 0));
-        }
-#pragma unroll
-        for (int k = 0; k < kBlk / 16; ++k) {
-          ptx::mma_f16_ss(tmem_base + Cfg::kColDK, desc_add(ds_mn, k * 2048), desc_add(q_m, k * 2048), idesc_t, (it > 0 || k > 0));
-        }
-        if (kPipe && it > 0) {
-          // dQ(it-1) has left tensor memory
-          if (!ptx::mbar_wait(dq_free, (it - 1) & 1, abort_flag)) break;
+        for (int k = 0; k < kBlk / 16; ++k)  // reduction over the 128 queries
+          ptx::mma_f16_ts(tmem_base + Cfg::kColDV, tmem_base + Cfg::kColP + (k >> 2) * Cfg::kPHalf + (k & 3) * 8,
+                          desc_add(do_m, k * 2048), idesc_kv, (it > 0 || k > 0));
+        ptx::tc_commit(&do_empty[it % DS]);
+        if (it + 1 < niter) {
+          if (!ptx::mbar_wait(&q_full[(it + 1) & 1], ((it + 1) >> 1) & 1, abort_flag)) break;
           ptx::tc_fence_after_sync();
+          issue_s(it + 1);   // the scores of `it` were read before p_full(it)
         }
+        if (!ptx::mbar_wait(ds_full, it & 1, abort_flag)) break;
+        if (!Cfg::kAlias && it > 0 && !ptx::mbar_wait(dq_free, (it - 1) & 1, abort_flag)) break;
+        ptx::tc_fence_after_sync();
 #pragma unroll
-        for (int k = 0; k < kBlk / 16; ++k) {  // reduction over the 128 keys
-          const uint32_t a_off = (k >> 2) * kChunkBytes + (k & 3) * 32;
-          ptx::mma_f16_ss(tmem_base + Cfg::kColDQ, desc_add(ds_kmaj, a_off), desc_add(k_mn, k * 2048), idesc_q, k > 0);
-        }
+        for (int k = 0; k < kBlk / 16; ++k)  // reduction over the 128 keys
+          ptx::mma_f16_ss(tmem_base + Cfg::kColDQ, desc_add(ds_mn, k * 2048), desc_add(k_mn, k * 2048), idesc_q, k > 0);
         ptx::tc_commit(dq_full);
-        ptx::tc_commit(&qdo_empty[st]);
-        if (!kPipe && it + 1 < niter) {
-          // dQ shares the S columns: the next S / dP wait for the flush of dQ(it)
-          if (!ptx::mbar_wait(&qdo_full[(it + 1) % S], ((it + 1) / S) & 1, abort_flag)) break;
-          if (!ptx::mbar_wait(dq_free, it & 1, abort_flag)) break;
+#pragma unroll
+        for (int k = 0; k < kBlk / 16; ++k)  // reduction over the 128 queries
+          ptx::mma_f16_ss(tmem_base + Cfg::kColDK, desc_add(ds_kmaj, (k >> 2) * kChunkBytes + (k & 3) * 32),
+                          desc_add(q_m, k * 2048), idesc_kv, (it > 0 || k > 0));
+        ptx::tc_commit(&q_empty[it & 1]);
+        if (it + 1 < niter) {
+          if (!ptx::mbar_wait(&do_full[(it + 1) % DS], ((it + 1) / DS) & 1, abort_flag)) break;
+          if (Cfg::kAlias && !ptx::mbar_wait(dq_free, it & 1, abort_flag)) break;
           ptx::tc_fence_after_sync();
-          issue_sdp(it + 1);
+          issue_dp(it + 1);
+        } else {
+          ptx::tc_commit(dkv_full);
         }
       }
     }
-  } else {
+  } else if (warp >= 8) {
+    // ------------------------------------------------------------ dQ
     const int quad = warp & 3;
-    const int half = (warp - 2) >> 2;
-    const int row = quad * 32 + lane;
-    const uint32_t lane_sel = static_cast<uint32_t>(quad * 32) << 16;
-    const float sc = p.scale * kLog2e;
-    uint8_t* p_smem = smem + Cfg::kP;
-    uint8_t* ds_smem = smem + Cfg::kDS;
-    bool ok = true;
-    // (lse, delta) of this thread's query row in iteration `it2`; rows past the end of the sequence get lse = +inf,
-    // which turns their probabilities into exact zeros
-    auto load_stats = [&](int it2, float& l, float& d) {
-      const int g2 = it2 / nq, i2 = jb + (it2 - g2 * nq);
-      const int q2 = i2 * kBlk + row;
-      const long long stat2 = (static_cast<long long>(b) * p.Hq + (hk * G + g2)) * p.T + q2;
-      // raw values: the conversion to base 2 happens where lse is used, so that nothing here waits for the loads
-      l = q2 < p.T ? p.lse[stat2] : INFINITY;
-      d = q2 < p.T ? p.delta[stat2] : 0.f;
-    };
-    // dQ of iteration `it2`, this warp's half of the head dimension, leaves tensor memory and is added to the fp32
-    // accumulator in HBM.  hd 64: through a swizzled shared-memory tile and one TMA reduce-add per half (rows past the
-    // end of the sequence are exact zeros, so adding them is harmless); hd 128: vector reductions from registers.
-    auto flush_dq = [&](int it2) {
-      const int g2 = it2 / nq, i2 = jb + (it2 - g2 * nq);
-      const int q2 = i2 * kBlk + row;
-      if constexpr (kPipe) {
-        uint8_t* stg = smem + Cfg::kDQ + half * (kBlk * 128);
-        const bool elected = (warp == 2 && lane == 0);
-        // the reduce-adds of the previous flush have finished reading the staging tiles
-        if (elected) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-        asm volatile("bar.sync 2, 256;" ::: "memory");
-        uint32_t r[32];
-        ptx::tmem_ld32(tmem_base + Cfg::kColDQ + lane_sel + half * 32, r);
-        ptx::tmem_ld_wait();
-        ptx::tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(dq_free);       // the dQ columns may be overwritten
+    const uint32_t t_dq = tmem_base + Cfg::kColDQ + (static_cast<uint32_t>(quad * 32) << 16);
+    uint8_t* stg = smem + Cfg::kDQ + quad * 8192;
+    auto stage = [&](const uint32_t (&r)[32], int piece) {
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
-          *reinterpret_cast<uint4*>(stg + row * 128 + ((u ^ (row & 7)) << 4)) =
-              make_uint4(r[u * 4], r[u * 4 + 1], r[u * 4 + 2], r[u * 4 + 3]);
+      for (int u = 0; u < 8; ++u)
+        *reinterpret_cast<uint4*>(stg + piece * 4096 + lane * 128 + ((u ^ (lane & 7)) << 4)) =
+            make_uint4(r[u * 4], r[u * 4 + 1], r[u * 4 + 2], r[u * 4 + 3]);
+    };
+    for (int it = 0; it < niter; ++it) {
+      const int g = it / nq, i = jb + (it - g * nq);
+      const int x = (hk * G + g) * HD, y = i * kBlk + quad * 32;
+      if (!ptx::mbar_wait(dq_full, it & 1, abort_flag)) break;
+      ptx::tc_fence_after_sync();
+      uint32_t r0[32], r1[32];
+      ptx::tmem_ld32(t_dq, r0);
+      ptx::tmem_ld32(t_dq + 32, r1);
+#pragma unroll
+      for (int c = 0; c < HD / 64; ++c) {
+        ptx::tmem_ld_wait();
+        if (c == HD / 64 - 1) {
+          ptx::tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(dq_free);       // the dQ columns may be overwritten
+        }
+        // the reduce-adds of the tiles staged before have finished reading them
+        if (lane == 0) ptx::bulk_wait_read<0>();
+        __syncwarp();
+        stage(r0, 0);
+        stage(r1, 1);
+        if (c + 1 < HD / 64) {
+          ptx::tmem_ld32(t_dq + (c + 1) * 64, r0);
+          ptx::tmem_ld32(t_dq + (c + 1) * 64 + 32, r1);
+        }
         ptx::fence_proxy_async_smem();
-        asm volatile("bar.sync 2, 256;" ::: "memory");
-        if (elected) {
-          const int x = (hk * G + g2) * HD, y = b * p.T + i2 * kBlk;
+        __syncwarp();
+        if (lane == 0 && y < p.T) {
 #pragma unroll
           for (int h2 = 0; h2 < 2; ++h2)
-            asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
+            asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
                              reinterpret_cast<uint64_t>(&tdq)),
-                         "r"(ptx::smem_u32(smem + Cfg::kDQ + h2 * (kBlk * 128))), "r"(x + h2 * 32), "r"(y)
+                         "r"(ptx::smem_u32(stg + h2 * 4096)), "r"(x + c * 64 + h2 * 32), "r"(y), "r"(b)
                          : "memory");
-          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          ptx::bulk_commit();
         }
-      } else {
-        float* dq_row = p.dq_accum + ((static_cast<long long>(b) * p.T + q2) * p.Hq + (hk * G + g2)) * HD;
-#pragma unroll 1
-        for (int c = half * (HD / 64); c < (half + 1) * (HD / 64); ++c) {
-          uint32_t r[32];
-          ptx::tmem_ld32(tmem_base + Cfg::kColDQ + lane_sel + c * 32, r);
-          ptx::tmem_ld_wait();
-          if (q2 < p.T) {
-#pragma unroll
-            for (int e = 0; e < 32; e += 4)
-              red_add_v4(dq_row + c * 32 + e, __uint_as_float(r[e]), __uint_as_float(r[e + 1]), __uint_as_float(r[e + 2]),
-                         __uint_as_float(r[e + 3]));
-          }
-        }
-        ptx::tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(dq_free);
       }
-    };
-    float pre_lse = 0.f, pre_dlt = 0.f;
-    if (niter > 0) load_stats(0, pre_lse, pre_dlt);
+    }
+    if (lane == 0) ptx::bulk_wait_all<0>();   // all reduce-adds done before the CTA exits
+  } else {
+    // ------------------------------------------------------------ element-wise
+    const int quad = warp & 3, half = warp >> 2;
+    const int row = quad * 32 + lane;                // key row
+    const uint32_t lane_sel = static_cast<uint32_t>(quad * 32) << 16;
+    const float sc = p.scale * kLog2e;
+    const uint32_t tS = tmem_base + Cfg::kColS + lane_sel + half * 64, tDP = tmem_base + Cfg::kColDP + lane_sel + half * 64;
+    const uint32_t tP = tmem_base + Cfg::kColP + lane_sel + half * Cfg::kPHalf;
+    uint8_t* ds_row = smem + Cfg::kDS + half * kChunkBytes + row * 128;
+    bool ok = true;
     for (int it = 0; it < niter; ++it) {
-      const int i = jb + (it % nq);
-      const int q_idx = i * kBlk + row;
-      const float lse2 = pre_lse, dlt = pre_dlt;       // requested one iteration ahead
-      if (it + 1 < niter) load_stats(it + 1, pre_lse, pre_dlt);
-      if (!ptx::mbar_wait(sdp_full, it & 1, abort_flag)) { ok = false; break; }
+      const float* nl = reinterpret_cast<const float*>(smem + Cfg::kStat) + (it & 1) * 2 * kBlk + half * 64;
+      const float* dl = nl + kBlk;
+      if (!ptx::mbar_wait(&stat_full[it & 1], (it >> 1) & 1, abort_flag)) { ok = false; break; }
+      if (!ptx::mbar_wait(s_full, it & 1, abort_flag)) { ok = false; break; }
       ptx::tc_fence_after_sync();
-      uint32_t s0[32], s1[32], d0[32], d1[32];
-      ptx::tmem_ld32(tmem_base + Cfg::kColS + lane_sel + half * 64, s0);
-      ptx::tmem_ld32(tmem_base + Cfg::kColS + lane_sel + half * 64 + 32, s1);
-      ptx::tmem_ld32(tmem_base + Cfg::kColDP + lane_sel + half * 64, d0);
-      ptx::tmem_ld32(tmem_base + Cfg::kColDP + lane_sel + half * 64 + 32, d1);
+      uint32_t pr[2][32];
+      ptx::tmem_ld32(tS, pr[0]);
+      ptx::tmem_ld32(tS + 32, pr[1]);
       ptx::tmem_ld_wait();
+      const bool diag = it % nq == 0;                // keys after the query get probability zero
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t pk[16];
+#pragma unroll
+        for (int e = 0; e < 32; e += 4) {
+          const float4 n4 = *reinterpret_cast<const float4*>(nl + c * 32 + e);
+          float x0, x1, x2, x3;
+          fma2(x0, x1, __uint_as_float(pr[c][e]), __uint_as_float(pr[c][e + 1]), sc, sc, n4.x, n4.y);
+          fma2(x2, x3, __uint_as_float(pr[c][e + 2]), __uint_as_float(pr[c][e + 3]), sc, sc, n4.z, n4.w);
+          x0 = ex2(x0); x1 = ex2(x1); x2 = ex2(x2); x3 = ex2(x3);
+          if (diag) {
+            const int q = half * 64 + c * 32 + e;
+            if (row > q) x0 = 0.f;
+            if (row > q + 1) x1 = 0.f;
+            if (row > q + 2) x2 = 0.f;
+            if (row > q + 3) x3 = 0.f;
+          }
+          pk[e / 2] = pack_bf16x2(x0, x1);
+          pk[e / 2 + 1] = pack_bf16x2(x2, x3);
+          pr[c][e] = __float_as_uint(x0); pr[c][e + 1] = __float_as_uint(x1);
+          pr[c][e + 2] = __float_as_uint(x2); pr[c][e + 3] = __float_as_uint(x3);
+        }
+        ptx::tmem_st16(tP + c * 16, pk);
+      }
+      ptx::tmem_st_wait();
       ptx::tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) ptx::mbar_arrive(sdp_free);       // S / dP columns may be overwritten
-      if (i == jb) {  // diagonal block: keys after the query get probability zero
-        const uint32_t ninf = __float_as_uint(-INFINITY);
-        const int kv0 = jb * kBlk + half * 64;
+      if (lane == 0) ptx::mbar_arrive(p_full);
+      if (!ptx::mbar_wait(dp_full, it & 1, abort_flag)) { ok = false; break; }
+      ptx::tc_fence_after_sync();
 #pragma unroll
-        for (int e = 0; e < 32; ++e) {
-          if (kv0 + e > q_idx) s0[e] = ninf;
-          if (kv0 + 32 + e > q_idx) s1[e] = ninf;
-        }
-      }
-      const float neg = -lse2 * kLog2e;
-      auto ew_chunk = [&](uint32_t (&rs)[32], uint32_t (&rd)[32], int c) {
-        uint32_t pk[16], dk_[16];
-#pragma unroll
-        for (int e = 0; e < 32; e += 2) {
-          const float p0 = ex2(fmaf(__uint_as_float(rs[e]), sc, neg));
-          const float p1 = ex2(fmaf(__uint_as_float(rs[e + 1]), sc, neg));
-          const float g0 = p0 * (__uint_as_float(rd[e]) - dlt) * p.scale;
-          const float g1 = p1 * (__uint_as_float(rd[e + 1]) - dlt) * p.scale;
-          pk[e >> 1] = pack_bf16x2(p0, p1);
-          dk_[e >> 1] = pack_bf16x2(g0, g1);
-        }
-        if (kPipe && c == 0 && it > 0) {
-          // MMA group 2 of the previous iteration must have finished reading P / dS (and produced dQ(it-1))
-          if (!ptx::mbar_wait(dq_full, (it - 1) & 1, abort_flag)) ok = false;
-          ptx::tc_fence_after_sync();
-        }
+      for (int c = 0; c < 2; ++c) {
+        uint32_t d[32];
+        ptx::tmem_ld32(tDP + c * 32, d);
+        ptx::tmem_ld_wait();
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          const uint32_t off = swz_off(row, half * 8 + c * 4 + u);
-          *reinterpret_cast<uint4*>(p_smem + off) = make_uint4(pk[u * 4], pk[u * 4 + 1], pk[u * 4 + 2], pk[u * 4 + 3]);
-          *reinterpret_cast<uint4*>(ds_smem + off) = make_uint4(dk_[u * 4], dk_[u * 4 + 1], dk_[u * 4 + 2], dk_[u * 4 + 3]);
+          uint32_t pk[4];
+#pragma unroll
+          for (int v = 0; v < 2; ++v) {
+            const int e = u * 8 + v * 4;
+            const float4 d4 = *reinterpret_cast<const float4*>(dl + c * 32 + e);
+            float x0, x1, x2, x3;
+            add2(x0, x1, __uint_as_float(d[e]), __uint_as_float(d[e + 1]), -d4.x, -d4.y);
+            add2(x2, x3, __uint_as_float(d[e + 2]), __uint_as_float(d[e + 3]), -d4.z, -d4.w);
+            mul2(x0, x1, x0, x1, __uint_as_float(pr[c][e]), __uint_as_float(pr[c][e + 1]));
+            mul2(x2, x3, x2, x3, __uint_as_float(pr[c][e + 2]), __uint_as_float(pr[c][e + 3]));
+            mul2(x0, x1, x0, x1, p.scale, p.scale);
+            mul2(x2, x3, x2, x3, p.scale, p.scale);
+            pk[v * 2] = pack_bf16x2(x0, x1);
+            pk[v * 2 + 1] = pack_bf16x2(x2, x3);
+          }
+          *reinterpret_cast<uint4*>(ds_row + (((c * 4 + u) ^ (row & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
         }
-      };
-      ew_chunk(s0, d0, 0);
-      if (!ok) break;
-      ew_chunk(s1, d1, 1);
+      }
       ptx::fence_proxy_async_smem();
       ptx::tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) ptx::mbar_arrive(pds_full);
-      if (kPipe) {
-        if (it > 0) flush_dq(it - 1);                   // underneath dV(it), dK(it)
-      } else {
-        // dQ shares the S columns: flush dQ(it) before the next S / dP may be issued
-        if (!ptx::mbar_wait(dq_full, it & 1, abort_flag)) { ok = false; break; }
-        ptx::tc_fence_after_sync();
-        flush_dq(it);
-      }
+      if (lane == 0) ptx::mbar_arrive(ds_full);
     }
-    if (kPipe && ok && niter > 0) {
-      ok = ptx::mbar_wait(dq_full, (niter - 1) & 1, abort_flag);
-      if (ok) {
-        ptx::tc_fence_after_sync();
-        flush_dq(niter - 1);
-      }
-    }
-    if (kPipe && warp == 2 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // all reduce-adds done
-    // The last dq_full arrival also covers every dV/dK accumulation issued before it.
+    if (ok) ok = ptx::mbar_wait(dkv_full, 0, abort_flag);
     const int kv_idx = jb * kBlk + row;
-    if (ok && niter > 0) {
+    if (ok) {
+      ptx::tc_fence_after_sync();
 #pragma unroll 1
       for (int which = 0; which < 2; ++which) {
         bf16* base = which == 0 ? p.dv : p.dk;
@@ -734,31 +795,43 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
 
   ptx::tc_fence_before_sync();
   __syncthreads();
-  if (warp == 1) {
+  if (warp == 13) {
     __syncwarp();
     ptx::tmem_dealloc(tmem_base, Cfg::kTmemCols);
   }
   if (threadIdx.x == 0 && *abort_flag) atomicExch(p.status, kStatusMbarTimeout);
 }
 
-// delta[b,h,t] = sum_d dO[b,t,h,d] * O[b,t,h,d]; one thread per (b,t,h) row.
+// delta[b,h,t] = sum_d dO[b,t,h,d] * O[b,t,h,d], and the fp32 dQ accumulator starts at zero.  hd / 8 neighbouring lanes
+// share a (b,t,h) row, 16 bytes of each operand per lane, so that every access of a warp is whole lines.
+template <int HD>
 __global__ void attn_delta_kernel(const bf16* __restrict__ d_o, const bf16* __restrict__ o, float* __restrict__ delta,
-                                  int B, int T, int H, int hd, long long do_stride_t, long long o_stride_t) {
-  const long long n = static_cast<long long>(B) * T * H;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+                                  float* __restrict__ dq_accum, int B, int T, int H, long long do_stride_t, long long o_stride_t) {
+  constexpr int L = HD / 8;
+  const long long n = static_cast<long long>(B) * T * H * L;
+  const long long n_up = (n + 31) / 32 * 32;   // whole warps take part in the shuffles
+  for (long long x = blockIdx.x * (long long)blockDim.x + threadIdx.x; x < n_up; x += (long long)gridDim.x * blockDim.x) {
+    const long long i = x / L;
+    const int d = static_cast<int>(x % L) * 8;
     const int h = static_cast<int>(i % H);
     const long long bt = i / H;
-    const bf16* a = d_o + bt * do_stride_t + h * hd;
-    const bf16* c = o + bt * o_stride_t + h * hd;
     float s = 0.f;
-    for (int d = 0; d < hd; d += 8) {
-      uint4 ua = *reinterpret_cast<const uint4*>(a + d), uc = *reinterpret_cast<const uint4*>(c + d);
-      float2 a0 = unpack_bf16x2(ua.x), a1 = unpack_bf16x2(ua.y), a2 = unpack_bf16x2(ua.z), a3 = unpack_bf16x2(ua.w);
-      float2 c0 = unpack_bf16x2(uc.x), c1 = unpack_bf16x2(uc.y), c2 = unpack_bf16x2(uc.z), c3 = unpack_bf16x2(uc.w);
-      s += a0.x * c0.x + a0.y * c0.y + a1.x * c1.x + a1.y * c1.y + a2.x * c2.x + a2.y * c2.y + a3.x * c3.x + a3.y * c3.y;
+    if (x < n) {
+      const uint4 ua = *reinterpret_cast<const uint4*>(d_o + bt * do_stride_t + h * HD + d);
+      const uint4 uc = *reinterpret_cast<const uint4*>(o + bt * o_stride_t + h * HD + d);
+      const float2 a0 = unpack_bf16x2(ua.x), a1 = unpack_bf16x2(ua.y), a2 = unpack_bf16x2(ua.z), a3 = unpack_bf16x2(ua.w);
+      const float2 c0 = unpack_bf16x2(uc.x), c1 = unpack_bf16x2(uc.y), c2 = unpack_bf16x2(uc.z), c3 = unpack_bf16x2(uc.w);
+      s = a0.x * c0.x + a0.y * c0.y + a1.x * c1.x + a1.y * c1.y + a2.x * c2.x + a2.y * c2.y + a3.x * c3.x + a3.y * c3.y;
+      float4* acc = reinterpret_cast<float4*>(dq_accum + i * HD + d);
+      acc[0] = make_float4(0.f, 0.f, 0.f, 0.f);
+      acc[1] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    const long long b = bt / T, t = bt - b * T;
-    delta[(b * H + h) * T + t] = s;
+#pragma unroll
+    for (int m = 1; m < L; m <<= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+    if (d == 0 && x < n) {
+      const long long b = bt / T, t = bt - b * T;
+      delta[(b * H + h) * T + t] = s;
+    }
   }
 }
 
@@ -828,24 +901,19 @@ static int attn_bwd_launch(const TitbAttnDesc* d, cudaStream_t st) {
     if (e != cudaSuccess) return static_cast<int>(e);
     attr_set[dev] = true;
   }
-  const uint64_t rows = static_cast<uint64_t>(d->B) * d->T;
   CUtensorMap tq, tk, tv, tdo, tdq;
-  if (!make_tmap_bf16_2d(&tq, d->q, static_cast<uint64_t>(d->Hq) * HD, rows, d->q_stride_t, 64, kBlk) ||
-      !make_tmap_bf16_2d(&tk, d->k, static_cast<uint64_t>(d->Hkv) * HD, rows, d->k_stride_t, 64, kBlk) ||
-      !make_tmap_bf16_2d(&tv, d->v, static_cast<uint64_t>(d->Hkv) * HD, rows, d->v_stride_t, 64, kBlk) ||
-      !make_tmap_bf16_2d(&tdo, d->d_o, static_cast<uint64_t>(d->Hq) * HD, rows, d->do_stride_t, 64, kBlk))
-    return TITB_ERR_TENSOR_MAP;
-  tdq = tq;  // placeholder where the kernel does not use it (hd 128)
-  if (!Cfg::kAliasDq && !make_tmap_f32_2d(&tdq, d->dq_accum, static_cast<uint64_t>(d->Hq) * HD, rows,
-                                          static_cast<uint64_t>(d->Hq) * HD, 32, kBlk))
+  const uint64_t B = d->B, T = d->T, wq = static_cast<uint64_t>(d->Hq) * HD, wkv = static_cast<uint64_t>(d->Hkv) * HD;
+  if (!make_tmap_tokens(&tq, d->q, 0, wq, T, B, d->q_stride_t, 64, kBlk) ||
+      !make_tmap_tokens(&tk, d->k, 0, wkv, T, B, d->k_stride_t, 64, kBlk) ||
+      !make_tmap_tokens(&tv, d->v, 0, wkv, T, B, d->v_stride_t, 64, kBlk) ||
+      !make_tmap_tokens(&tdo, d->d_o, 0, wq, T, B, d->do_stride_t, 64, kBlk) ||
+      !make_tmap_tokens(&tdq, d->dq_accum, 1, wq, T, B, wq, 32, 32))
     return TITB_ERR_TENSOR_MAP;
   const long long nrows = static_cast<long long>(d->B) * d->T * d->Hq;
-  int blocks = static_cast<int>((nrows + 255) / 256);
-  if (blocks > device_sm_count() * 8) blocks = device_sm_count() * 8;
-  attn_delta_kernel<<<blocks, 256, 0, st>>>(static_cast<const bf16*>(d->d_o), static_cast<const bf16*>(d->o), d->delta,
-                                            d->B, d->T, d->Hq, HD, d->do_stride_t, d->o_stride_t);
-  cudaError_t e = cudaMemsetAsync(d->dq_accum, 0, sizeof(float) * nrows * HD, st);
-  if (e != cudaSuccess) return static_cast<int>(e);
+  const long long delta_blocks = (nrows * (HD / 8) + 255) / 256, delta_max = device_sm_count() * 16LL;
+  attn_delta_kernel<HD><<<static_cast<int>(delta_blocks < delta_max ? delta_blocks : delta_max), 256, 0, st>>>(
+      static_cast<const bf16*>(d->d_o), static_cast<const bf16*>(d->o), d->delta, d->dq_accum, d->B, d->T, d->Hq,
+      d->do_stride_t, d->o_stride_t);
   AttnArgs a{};
   a.B = d->B; a.T = d->T; a.Hq = d->Hq; a.Hkv = d->Hkv; a.hd = HD;
   a.scale = d->scale;
@@ -853,8 +921,8 @@ static int attn_bwd_launch(const TitbAttnDesc* d, cudaStream_t st) {
   a.dk = static_cast<bf16*>(d->dk); a.dv = static_cast<bf16*>(d->dv);
   a.dk_stride_t = d->dk_stride_t; a.dv_stride_t = d->dv_stride_t;
   a.status = titb_status_ptr();
-  dim3 grid((d->T + kBlk - 1) / kBlk, d->Hkv, d->B);
-  attn_bwd_kernel<HD><<<grid, 320, Cfg::kSmem, st>>>(tq, tk, tv, tdo, tdq, a);
+  dim3 grid(static_cast<unsigned>(d->Hkv) * d->B, (d->T + kBlk - 1) / kBlk);
+  attn_bwd_kernel<HD><<<grid, kBwdThreads, Cfg::kSmem, st>>>(tq, tk, tv, tdo, tdq, a);
   const long long bt = static_cast<long long>(d->B) * d->T;
   const int width = d->Hq * HD;
   int cb = static_cast<int>((bt * (width / 8) + 255) / 256);

@@ -1193,6 +1193,28 @@ bool make_tmap_f32_2d(CUtensorMap* m, const void* base, uint64_t inner, uint64_t
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// [B, T, width] tokens with `ld` elements between tokens and T * ld between sequences, bf16 or fp32; a box is box_width
+// columns (128 bytes) of box_tokens tokens of ONE sequence: what a tile has past the end of its sequence reads as zero
+// and is not written.
+bool make_tmap_tokens(CUtensorMap* m, const void* base, int fp32, uint64_t width, uint64_t T, uint64_t B, uint64_t ld,
+                      uint32_t box_width, uint32_t box_tokens) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn) return false;
+  static thread_local bool ctx_bound = false;   // see make_tmap_bf16_2d
+  if (!ctx_bound) {
+    cudaFree(nullptr);
+    ctx_bound = true;
+  }
+  const uint64_t elem = fp32 ? 4 : 2;
+  cuuint64_t dims[3] = {width, T, B};
+  cuuint64_t strides[2] = {ld * elem, T * ld * elem};
+  cuuint32_t box[3] = {box_width, box_tokens, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return fn(m, fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims,
+            strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 static int g_no_tma_store = 0;  // set by titb_gemm_set_tma_store(0): A/B switch for the epilogue store path
 
 // Estimated duration of a GEMM for a tile width and a split-K factor, in units of one k-block (64 deep) of a
