@@ -645,7 +645,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
     for (int it = 0; it < niter; ++it) {
       const int g = it / nq, i = jb + (it - g * nq);
       const int x = (hk * G + g) * HD, y = i * kBlk + quad * 32;
-      if (!ptx::mbar_wait(dq_full, it & 1, abort_flag)) break;
+      if (!ptx::mbar_wait_warp(dq_full, it & 1, abort_flag)) break;
       ptx::tc_fence_after_sync();
       uint32_t r0[32], r1[32];
       ptx::tmem_ld32(t_dq, r0);
@@ -694,8 +694,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
     for (int it = 0; it < niter; ++it) {
       const float* nl = reinterpret_cast<const float*>(smem + Cfg::kStat) + (it & 1) * 2 * kBlk + half * 64;
       const float* dl = nl + kBlk;
-      if (!ptx::mbar_wait(&stat_full[it & 1], (it >> 1) & 1, abort_flag)) { ok = false; break; }
-      if (!ptx::mbar_wait(s_full, it & 1, abort_flag)) { ok = false; break; }
+      if (!ptx::mbar_wait_warp(&stat_full[it & 1], (it >> 1) & 1, abort_flag)) { ok = false; break; }
+      if (!ptx::mbar_wait_warp(s_full, it & 1, abort_flag)) { ok = false; break; }
       ptx::tc_fence_after_sync();
       uint32_t pr[2][32];
       ptx::tmem_ld32(tS, pr[0]);
@@ -730,7 +730,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
       ptx::tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(p_full);
-      if (!ptx::mbar_wait(dp_full, it & 1, abort_flag)) { ok = false; break; }
+      if (!ptx::mbar_wait_warp(dp_full, it & 1, abort_flag)) { ok = false; break; }
       ptx::tc_fence_after_sync();
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
@@ -762,7 +762,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(ds_full);
     }
-    if (ok) ok = ptx::mbar_wait(dkv_full, 0, abort_flag);
+    if (ok) ok = ptx::mbar_wait_warp(dkv_full, 0, abort_flag);
     const int kv_idx = jb * kBlk + row;
     if (ok) {
       ptx::tc_fence_after_sync();

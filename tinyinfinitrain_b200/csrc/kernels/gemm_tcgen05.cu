@@ -248,6 +248,136 @@ __device__ __forceinline__ void epilogue_row32(const GemmArgs& p, float (&v)[32]
   }
 }
 
+// One warp's 32 rows x 64 columns of a tile on their way out: `v` holds this lane's row.  The piece goes through the
+// warp's own staging tiles and its own TMA stores, so the four epilogue warps never wait for one another (with one
+// 128-row store per chunk they met at two barriers per 64 columns).  `buf` counts the pieces this warp has staged.
+struct WarpOut {
+  uint8_t* out;   // 4 KB staging tile of the result
+  uint8_t* aux;   // 4 KB: second result tile, or the auxiliary operand / result of the epilogue
+  int buf;
+};
+
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, const void* smem, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
+                   reinterpret_cast<uint64_t>(m)), "r"(ptx::smem_u32(smem)), "r"(x), "r"(y)
+               : "memory");
+}
+__device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* m, const void* smem, int x, int y) {
+  asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
+                   reinterpret_cast<uint64_t>(m)), "r"(ptx::smem_u32(smem)), "r"(x), "r"(y)
+               : "memory");
+}
+
+// fp32 results, 32 columns at a time: the two staging tiles alternate.
+__device__ __forceinline__ void put_f32(const GemmArgs& p, const CUtensorMap* tout, WarpOut& w, const float* v, int row0,
+                                        int col0, int lane) {
+  uint8_t* stg = (w.buf++ & 1) ? w.aux : w.out;
+  // the copy issued two pieces ago has finished reading this staging tile
+  if (ptx::elect_one()) ptx::bulk_wait_read<1>();
+  __syncwarp();
+#pragma unroll
+  for (int u = 0; u < 8; ++u)
+    *reinterpret_cast<float4*>(stg + lane * 128 + ((u ^ (lane & 7)) << 4)) =
+        make_float4(v[u * 4], v[u * 4 + 1], v[u * 4 + 2], v[u * 4 + 3]);
+  ptx::fence_proxy_async_smem();
+  __syncwarp();
+  if (ptx::elect_one()) {
+    if (p.f32_red) tma_reduce_add_2d(tout, stg, col0, row0);
+    else tma_store_2d(tout, stg, col0, row0);
+    ptx::bulk_commit();
+  }
+}
+
+// bf16 results, 64 columns at a time: bias, activation, residual, then the store.  `aux_row`: this lane's row of the
+// auxiliary operand when it comes through the staging tile (aux_tma_load), otherwise it is read from memory.
+__device__ __forceinline__ void put_bf16(const GemmArgs& p, const CUtensorMap* tout, const CUtensorMap* taux, WarpOut& w,
+                                         float (&v)[64], const uint4 (&aux_row)[8], int row0, int col0, int lane) {
+  const long long row = row0 + lane;
+  const bool full_cols = (col0 + 64 <= p.N);
+  if (p.bias != nullptr && (p.epi == TITB_EPI_BIAS || p.epi == TITB_EPI_BIAS_GELU || p.epi == TITB_EPI_BIAS_RESIDUAL)) {
+    if (full_cols) {
+#pragma unroll
+      for (int j = 0; j < 64; j += 8) {
+        const uint4 u = *reinterpret_cast<const uint4*>(p.bias + col0 + j);
+        const float2 f0 = unpack_bf16x2(u.x), f1 = unpack_bf16x2(u.y), f2 = unpack_bf16x2(u.z), f3 = unpack_bf16x2(u.w);
+        v[j] += f0.x; v[j + 1] += f0.y; v[j + 2] += f1.x; v[j + 3] += f1.y;
+        v[j + 4] += f2.x; v[j + 5] += f2.y; v[j + 6] += f3.x; v[j + 7] += f3.y;
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 64; ++j) if (col0 + j < p.N) v[j] += __bfloat162float(p.bias[col0 + j]);
+    }
+  }
+  uint32_t aux_pk[32];
+  if (p.epi == TITB_EPI_BIAS_GELU) {
+#pragma unroll
+    for (int j = 0; j < 64; j += 2) {
+      aux_pk[j >> 1] = pack_bf16x2(v[j], v[j + 1]);
+      const float2 pr = unpack_bf16x2(aux_pk[j >> 1]);  // activation of the stored (rounded) pre-activation
+      v[j] = gelu_fast(pr.x);
+      v[j + 1] = gelu_fast(pr.y);
+    }
+  } else if (p.aux_tma_load) {
+    // out-of-range rows / columns of the aux tile were zero-filled by the TMA load
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const float2 f0 = unpack_bf16x2(aux_row[u].x), f1 = unpack_bf16x2(aux_row[u].y), f2 = unpack_bf16x2(aux_row[u].z),
+                   f3 = unpack_bf16x2(aux_row[u].w);
+      const float a8[8] = {f0.x, f0.y, f1.x, f1.y, f2.x, f2.y, f3.x, f3.y};
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        v[u * 8 + e] = (p.epi == TITB_EPI_DGELU) ? v[u * 8 + e] * gelu_grad_fast(a8[e]) : v[u * 8 + e] + a8[e];
+    }
+  } else if ((p.epi == TITB_EPI_DGELU || p.epi == TITB_EPI_BIAS_RESIDUAL) && p.aux_in != nullptr && row < p.M) {
+    const bf16* ai = p.aux_in + row * p.ld_aux_in + col0;
+    if (full_cols) {
+#pragma unroll
+      for (int j = 0; j < 64; j += 8) {
+        const uint4 u = *reinterpret_cast<const uint4*>(ai + j);
+        const float2 f0 = unpack_bf16x2(u.x), f1 = unpack_bf16x2(u.y), f2 = unpack_bf16x2(u.z), f3 = unpack_bf16x2(u.w);
+        const float a8[8] = {f0.x, f0.y, f1.x, f1.y, f2.x, f2.y, f3.x, f3.y};
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[j + e] = (p.epi == TITB_EPI_DGELU) ? v[j + e] * gelu_grad_fast(a8[e]) : v[j + e] + a8[e];
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 64; ++j) {
+        if (col0 + j < p.N) {
+          const float a1 = __bfloat162float(ai[j]);
+          v[j] = (p.epi == TITB_EPI_DGELU) ? v[j] * gelu_grad_fast(a1) : v[j] + a1;
+        }
+      }
+    }
+  }
+  const bool two_results = p.epi == TITB_EPI_BIAS_GELU && p.aux_out != nullptr;
+  // without a second result or operand both staging tiles take results in turn
+  const bool alternate = !two_results && !p.aux_tma_load;
+  uint8_t* stg = (alternate && (w.buf & 1)) ? w.aux : w.out;
+  ++w.buf;
+  if (ptx::elect_one()) {   // the store that used this staging tile has finished reading it
+    if (alternate) ptx::bulk_wait_read<1>();
+    else ptx::bulk_wait_read<0>();
+  }
+  __syncwarp();
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    const uint32_t off = static_cast<uint32_t>(lane * 128 + ((u ^ (lane & 7)) << 4));
+    *reinterpret_cast<uint4*>(stg + off) =
+        make_uint4(pack_bf16x2(v[u * 8], v[u * 8 + 1]), pack_bf16x2(v[u * 8 + 2], v[u * 8 + 3]),
+                   pack_bf16x2(v[u * 8 + 4], v[u * 8 + 5]), pack_bf16x2(v[u * 8 + 6], v[u * 8 + 7]));
+    if (two_results)
+      *reinterpret_cast<uint4*>(w.aux + off) =
+          make_uint4(aux_pk[u * 4], aux_pk[u * 4 + 1], aux_pk[u * 4 + 2], aux_pk[u * 4 + 3]);
+  }
+  ptx::fence_proxy_async_smem();
+  __syncwarp();
+  if (ptx::elect_one()) {
+    tma_store_2d(tout, stg, col0, row0);
+    if (two_results) tma_store_2d(taux, w.aux, col0, row0);
+    ptx::bulk_commit();
+  }
+}
+
 struct TileCoord { int m0, n0, split, mblk; };
 
 __device__ __forceinline__ TileCoord tile_coord(const GemmArgs& p, int tile, int tiles_m, int tiles_n, int bn,
@@ -590,15 +720,15 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
   uint64_t* empty = full + kStages;
   uint64_t* acc_full = empty + kStages;
   uint64_t* acc_empty = acc_full + 2;
-  uint64_t* aux_bar = acc_empty + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(aux_bar + 1);
+  uint64_t* aux_bar = acc_empty + 2;   // one per epilogue warp
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(aux_bar + 4);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int warp = ptx::warp_index();
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    ptx::mbar_init(aux_bar, 1);
+    for (int w = 0; w < 4; ++w) ptx::mbar_init(&aux_bar[w], 1);
     for (int s = 0; s < kStages; ++s) {
       ptx::mbar_init(&full[s], 1);
       ptx::mbar_init(&empty[s], 1);
@@ -787,7 +917,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
         const int m0 = tc.m0, n0 = tc.n0;
         const int buf = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
-        if (!ptx::mbar_wait(&acc_full[buf], acc_phase, abort_flag)) break;
+        if (!ptx::mbar_wait_warp(&acc_full[buf], acc_phase, abort_flag)) break;
         ptx::tc_fence_after_sync();
         const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + buf * Cfg::kAccStride;
         const int owner = m0 / p.coll.rows_per_rank;
@@ -842,232 +972,108 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
       }
       rs_reduce_phase(p, tiles_n, cta, ncta, tid);
     } else if (p.tma_store == 2) {
-      // fp32 outputs (weight gradients): 32 columns at a time -> registers -> swizzled shared-memory tile -> one TMA
-      // store, or one TMA reduce-add when the tile is a split-K partial or accumulates into the output.  The two
-      // staging tiles alternate, so the copy of chunk c overlaps the staging of chunk c + 1.
-      const int trow = quad * 32 + lane;
-      const bool elected = (warp == 2 && lane == 0);
-      int gchunk = 0;
+      // fp32 outputs (weight gradients): registers -> the warp's swizzled staging tile -> one TMA store, or one TMA
+      // reduce-add when the tile is a split-K partial or accumulates into the output.
+      WarpOut wo{stage_out + (warp - 2) * 4096, stage_aux + (warp - 2) * 4096, 0};
       for (int rnd = walk.first_round(), tile; (tile = walk.tile(rnd)) < num_tiles; ++rnd, ++it) {
         const TileCoord tc = tile_coord(p, tile, tiles_m, tiles_n, BN, kTileM, row_off);
         const int m0 = tc.m0, n0 = tc.n0;
         const int buf = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
-        if (!ptx::mbar_wait(&acc_full[buf], acc_phase, abort_flag)) break;
+        if (!ptx::mbar_wait_warp(&acc_full[buf], acc_phase, abort_flag)) break;
         ptx::tc_fence_after_sync();
         const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + buf * Cfg::kAccStride;
 #pragma unroll 1
         for (int c = 0; c < BN / 32; ++c) {
           const int col0 = n0 + c * 32;
           const bool last = (c == BN / 32 - 1);
-          if (col0 >= p.N) {  // whole chunk is padding
-            if (last) {
-              ptx::tc_fence_before_sync();
-              __syncwarp();
-              if (lane == 0) release_acc(buf);
-            }
-            continue;
-          }
           uint32_t r[32];
-          ptx::tmem_ld32(t_row + c * 32, r);
-          ptx::tmem_ld_wait();
+          if (col0 < p.N) {
+            ptx::tmem_ld32(t_row + c * 32, r);
+            ptx::tmem_ld_wait();
+          }
           if (last) {  // accumulator fully read: the MMA warp may reuse this TMEM buffer
             ptx::tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) release_acc(buf);
           }
-          if (p.alpha != nullptr) {
-            const float al = *p.alpha;
+          if (col0 >= p.N || m0 + quad * 32 >= p.M) continue;   // nothing but padding
+          const float al = p.alpha != nullptr ? *p.alpha : 1.f;
+          float v[32];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * al);
-          }
-          uint8_t* stg = (gchunk & 1) ? stage_aux : stage_out;
-          // the copy issued two chunks ago has finished reading this staging tile
-          if (elected) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-          asm volatile("bar.sync 1, 128;" ::: "memory");
-#pragma unroll
-          for (int u = 0; u < 8; ++u)
-            *reinterpret_cast<uint4*>(stg + trow * 128 + ((u ^ (trow & 7)) << 4)) =
-                make_uint4(r[u * 4], r[u * 4 + 1], r[u * 4 + 2], r[u * 4 + 3]);
-          ptx::fence_proxy_async_smem();
-          asm volatile("bar.sync 1, 128;" ::: "memory");
-          if (elected) {
-            if (p.f32_red)
-              asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
-                               reinterpret_cast<uint64_t>(&tma_out)),
-                           "r"(ptx::smem_u32(stg)), "r"(col0), "r"(m0)
-                           : "memory");
-            else
-              asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
-                               reinterpret_cast<uint64_t>(&tma_out)),
-                           "r"(ptx::smem_u32(stg)), "r"(col0), "r"(m0)
-                           : "memory");
-            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-          }
-          ++gchunk;
+          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * al;
+          put_f32(p, &tma_out, wo, v, m0 + quad * 32, col0, lane);
         }
       }
-      if (elected) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // all copies done before the CTA exits
+      if (ptx::elect_one()) ptx::bulk_wait_read<0>();  // the staging tiles must outlive the copies
     } else if (p.tma_store) {
-      // bf16 outputs: 64 columns at a time -> registers -> swizzled shared-memory tile -> one TMA
-      // store per tile chunk (full 128-byte lines instead of one 16-byte piece per thread and row).
-      const int trow = quad * 32 + lane;
-      const bool elected = (warp == 2 && lane == 0);
-      // Residual / pre-activation tiles are fetched one chunk ahead by TMA into the aux staging tile.
+      WarpOut wo{stage_out + (warp - 2) * 4096, stage_aux + (warp - 2) * 4096, 0};
+      // Residual / pre-activation tiles are fetched one chunk ahead by TMA into the warp's aux staging tile.
       constexpr int kChunksPerTile = BN / 64;
+      uint64_t* my_aux_bar = &aux_bar[warp - 2];
       const int my_tiles = cta < num_tiles ? (num_tiles - cta + ncta - 1) / ncta : 0;
       const int total_chunks = my_tiles * kChunksPerTile;
       auto issue_aux_load = [&](int g) {  // g: running chunk index over this CTA's tiles
         const int t_local = g / kChunksPerTile;
         const TileCoord t2 = tile_coord(p, cta + t_local * ncta, tiles_m, tiles_n, BN, kTileM, row_off);
-        ptx::mbar_expect_tx(aux_bar, kBM * 128);
-        ptx::tma_load_2d(stage_aux, &tma_aux, aux_bar, t2.n0 + (g % kChunksPerTile) * 64, t2.m0);
+        ptx::mbar_expect_tx(my_aux_bar, 4096);
+        ptx::tma_load_2d(wo.aux, &tma_aux, my_aux_bar, t2.n0 + (g % kChunksPerTile) * 64, t2.m0 + quad * 32);
       };
       int gchunk = 0;
-      if (p.aux_tma_load && elected && total_chunks > 0) issue_aux_load(0);
+      if (p.aux_tma_load && total_chunks > 0 && ptx::elect_one()) issue_aux_load(0);
       for (int rnd = walk.first_round(), tile; (tile = walk.tile(rnd)) < num_tiles; ++rnd, ++it) {
         const TileCoord tc = tile_coord(p, tile, tiles_m, tiles_n, BN, kTileM, row_off);
         const int m0 = tc.m0, n0 = tc.n0;
         const int buf = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
-        if (!ptx::mbar_wait(&acc_full[buf], acc_phase, abort_flag)) break;
+        // the bias of this tile is on its way to L1 while the main loop runs
+        if (p.bias != nullptr && lane < BN / 64 && n0 + lane * 64 < p.N)
+          asm volatile("prefetch.global.L1 [%0];" ::"l"(p.bias + n0 + lane * 64));
+        if (!ptx::mbar_wait_warp(&acc_full[buf], acc_phase, abort_flag)) break;
         ptx::tc_fence_after_sync();
-        const long long row = m0 + trow;
         const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + buf * Cfg::kAccStride;
 #pragma unroll 1
         for (int c = 0; c < BN / 64; ++c) {
           const int col0 = n0 + c * 64;
           uint4 aux_row[8];
           if (p.aux_tma_load) {
-            // chunk `gchunk` of the aux operand has landed; copy this thread's row out and prefetch the next
-            const bool got = ptx::mbar_wait(aux_bar, gchunk & 1, abort_flag);
-            if (got) {
+            // chunk `gchunk` of the aux operand has landed; copy this lane's row out and prefetch the next
+            if (ptx::mbar_wait(my_aux_bar, gchunk & 1, abort_flag)) {
 #pragma unroll
               for (int u = 0; u < 8; ++u)
-                aux_row[u] = *reinterpret_cast<const uint4*>(stage_aux + trow * 128 + ((u ^ (trow & 7)) << 4));
+                aux_row[u] = *reinterpret_cast<const uint4*>(wo.aux + lane * 128 + ((u ^ (lane & 7)) << 4));
             }
-            asm volatile("bar.sync 1, 128;" ::: "memory");
+            __syncwarp();
             ++gchunk;
-            if (elected && gchunk < total_chunks) issue_aux_load(gchunk);
-          }
-          if (col0 >= p.N) {  // whole chunk is padding: nothing to read or store, but keep the barriers in step
-            if (c == BN / 64 - 1) {
-              ptx::tc_fence_before_sync();
-              __syncwarp();
-              if (lane == 0) release_acc(buf);
-            }
-            continue;
+            if (gchunk < total_chunks && ptx::elect_one()) issue_aux_load(gchunk);
           }
           uint32_t r0[32], r1[32];
-          ptx::tmem_ld32(t_row + c * 64, r0);
-          ptx::tmem_ld32(t_row + c * 64 + 32, r1);
-          ptx::tmem_ld_wait();
+          if (col0 < p.N) {
+            ptx::tmem_ld32(t_row + c * 64, r0);
+            ptx::tmem_ld32(t_row + c * 64 + 32, r1);
+            ptx::tmem_ld_wait();
+          }
           if (c == BN / 64 - 1) {  // accumulator fully read: the MMA warp may reuse this TMEM buffer
             ptx::tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) release_acc(buf);
           }
+          if (col0 >= p.N || m0 + quad * 32 >= p.M) continue;   // nothing but padding
+          const float al = p.alpha != nullptr ? *p.alpha : 1.f;
           float v[64];
 #pragma unroll
-          for (int j = 0; j < 32; ++j) { v[j] = __uint_as_float(r0[j]); v[32 + j] = __uint_as_float(r1[j]); }
-          if (p.alpha != nullptr) {
-            const float al = *p.alpha;
-#pragma unroll
-            for (int j = 0; j < 64; ++j) v[j] *= al;
-          }
-          const bool full_cols = (col0 + 64 <= p.N);
-          if (p.bias != nullptr && (p.epi == TITB_EPI_BIAS || p.epi == TITB_EPI_BIAS_GELU || p.epi == TITB_EPI_BIAS_RESIDUAL)) {
-            if (full_cols) {
-#pragma unroll
-              for (int j = 0; j < 64; j += 8) {
-                const uint4 u = *reinterpret_cast<const uint4*>(p.bias + col0 + j);
-                const float2 f0 = unpack_bf16x2(u.x), f1 = unpack_bf16x2(u.y), f2 = unpack_bf16x2(u.z), f3 = unpack_bf16x2(u.w);
-                v[j] += f0.x; v[j + 1] += f0.y; v[j + 2] += f1.x; v[j + 3] += f1.y;
-                v[j + 4] += f2.x; v[j + 5] += f2.y; v[j + 6] += f3.x; v[j + 7] += f3.y;
-              }
-            } else {
-#pragma unroll
-              for (int j = 0; j < 64; ++j) if (col0 + j < p.N) v[j] += __bfloat162float(p.bias[col0 + j]);
-            }
-          }
-          uint32_t aux_pk[32];
-          if (p.epi == TITB_EPI_BIAS_GELU) {
-#pragma unroll
-            for (int j = 0; j < 64; j += 2) {
-              aux_pk[j >> 1] = pack_bf16x2(v[j], v[j + 1]);
-              const float2 pr = unpack_bf16x2(aux_pk[j >> 1]);  // activation of the stored (rounded) pre-activation
-              v[j] = gelu_fast(pr.x);
-              v[j + 1] = gelu_fast(pr.y);
-            }
-          } else if (p.aux_tma_load) {
-            // out-of-range rows / columns of the aux tile were zero-filled by the TMA load
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-              const float2 f0 = unpack_bf16x2(aux_row[u].x), f1 = unpack_bf16x2(aux_row[u].y), f2 = unpack_bf16x2(aux_row[u].z),
-                           f3 = unpack_bf16x2(aux_row[u].w);
-              const float a8[8] = {f0.x, f0.y, f1.x, f1.y, f2.x, f2.y, f3.x, f3.y};
-#pragma unroll
-              for (int e = 0; e < 8; ++e)
-                v[u * 8 + e] = (p.epi == TITB_EPI_DGELU) ? v[u * 8 + e] * gelu_grad_fast(a8[e]) : v[u * 8 + e] + a8[e];
-            }
-          } else if ((p.epi == TITB_EPI_DGELU || p.epi == TITB_EPI_BIAS_RESIDUAL) && p.aux_in != nullptr && row < p.M) {
-            const bf16* ai = p.aux_in + row * p.ld_aux_in + col0;
-            if (full_cols) {
-#pragma unroll
-              for (int j = 0; j < 64; j += 8) {
-                const uint4 u = *reinterpret_cast<const uint4*>(ai + j);
-                const float2 f0 = unpack_bf16x2(u.x), f1 = unpack_bf16x2(u.y), f2 = unpack_bf16x2(u.z), f3 = unpack_bf16x2(u.w);
-                const float a8[8] = {f0.x, f0.y, f1.x, f1.y, f2.x, f2.y, f3.x, f3.y};
-#pragma unroll
-                for (int e = 0; e < 8; ++e) v[j + e] = (p.epi == TITB_EPI_DGELU) ? v[j + e] * gelu_grad_fast(a8[e]) : v[j + e] + a8[e];
-              }
-            } else {
-#pragma unroll
-              for (int j = 0; j < 64; ++j) {
-                if (col0 + j < p.N) {
-                  const float a1 = __bfloat162float(ai[j]);
-                  v[j] = (p.epi == TITB_EPI_DGELU) ? v[j] * gelu_grad_fast(a1) : v[j] + a1;
-                }
-              }
-            }
-          }
-          // the previous chunk's TMA store must have finished reading the staging tiles
-          if (elected) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-          asm volatile("bar.sync 1, 128;" ::: "memory");
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const uint32_t off = static_cast<uint32_t>(trow * 128 + ((u ^ (trow & 7)) << 4));
-            *reinterpret_cast<uint4*>(stage_out + off) =
-                make_uint4(pack_bf16x2(v[u * 8], v[u * 8 + 1]), pack_bf16x2(v[u * 8 + 2], v[u * 8 + 3]),
-                           pack_bf16x2(v[u * 8 + 4], v[u * 8 + 5]), pack_bf16x2(v[u * 8 + 6], v[u * 8 + 7]));
-            if (p.epi == TITB_EPI_BIAS_GELU && p.aux_out != nullptr)
-              *reinterpret_cast<uint4*>(stage_aux + off) =
-                  make_uint4(aux_pk[u * 4], aux_pk[u * 4 + 1], aux_pk[u * 4 + 2], aux_pk[u * 4 + 3]);
-          }
-          ptx::fence_proxy_async_smem();
-          asm volatile("bar.sync 1, 128;" ::: "memory");
-          if (elected) {
-            asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
-                             reinterpret_cast<uint64_t>(&tma_out)),
-                         "r"(ptx::smem_u32(stage_out)), "r"(col0), "r"(m0)
-                         : "memory");
-            if (p.epi == TITB_EPI_BIAS_GELU && p.aux_out != nullptr)
-              asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
-                               reinterpret_cast<uint64_t>(&tma_aux)),
-                           "r"(ptx::smem_u32(stage_aux)), "r"(col0), "r"(m0)
-                           : "memory");
-            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-          }
+          for (int j = 0; j < 32; ++j) { v[j] = __uint_as_float(r0[j]) * al; v[32 + j] = __uint_as_float(r1[j]) * al; }
+          put_bf16(p, &tma_out, &tma_aux, wo, v, aux_row, m0 + quad * 32, col0, lane);
         }
       }
-      if (elected) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // all stores done before the CTA exits
+      if (ptx::elect_one()) ptx::bulk_wait_read<0>();  // the staging tiles must outlive the stores
     } else
     for (int rnd = walk.first_round(), tile; (tile = walk.tile(rnd)) < num_tiles; ++rnd, ++it) {
       const TileCoord tc = tile_coord(p, tile, tiles_m, tiles_n, BN, kTileM, row_off);
       const int split = tc.split, m0 = tc.m0, n0 = tc.n0;
       const int buf = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1;
-      if (!ptx::mbar_wait(&acc_full[buf], acc_phase, abort_flag)) break;
+      if (!ptx::mbar_wait_warp(&acc_full[buf], acc_phase, abort_flag)) break;
       ptx::tc_fence_after_sync();
       const long long row = m0 + quad * 32 + lane;
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + buf * Cfg::kAccStride;
@@ -1217,13 +1223,16 @@ bool make_tmap_tokens(CUtensorMap* m, const void* base, int fp32, uint64_t width
 
 static int g_no_tma_store = 0;  // set by titb_gemm_set_tma_store(0): A/B switch for the epilogue store path
 
-// Estimated duration of a GEMM for a tile width and a split-K factor, in units of one k-block (64 deep) of a
-// lightly loaded SM (about 0.4 us, measured: the same for 128-, 192- and 256-wide tiles when few CTAs run).  When
-// most SMs are busy the operand traffic out of L2 sets the pace and a k-block costs more, in proportion to the
-// bytes it loads ((128 + BN) x 64 x 2): about 1.7 units for a 128 x 256 tile on a full machine.  The epilogue of
-// the last tile of a CTA is exposed (earlier ones overlap the next main loop); a split adds the zero fill of the
-// output and the contention of the partial tiles' reduce-adds.
+// Estimated duration (us) of a GEMM for a tile width and a split-K factor.  The constants are a least-regret fit to 183
+// shapes of GPT-2 124M / XL and LLaMA-3 1B / 8B layers at 256 to 8192 tokens (forward, input and weight gradients, each
+// timed with every width and split): the choices are 0.4 % off the fastest configuration on average, where constants from
+// before MMAs were issued by an elected lane, when every width took the same time per k-block, were 9.7 % off.
+//   k-block   how long 64 reduction steps of a tile take: the MMAs, or on a full machine the operand bytes out of L2
+//   fixed     launch, pipeline fill, the last epilogue
+//   epilogue  what the next main loop does not hide of an epilogue
+//   a split   zero fill of the output, and the reduce-adds of the partial tiles
 static double plan_cost(int M, int N, int K, int bn, int splits, int sms) {
+  const double k_block = bn == 128 ? 0.224 : bn == 192 ? 0.241 : 0.325, fixed = bn == 128 ? 5.0 : bn == 192 ? 6.1 : 5.6;
   const long long tm = (M + kBM - 1) / kBM, tn = (N + bn - 1) / bn;
   const int kb = (K + kBK - 1) / kBK;
   const int kb_per = (kb + splits - 1) / splits;
@@ -1231,24 +1240,24 @@ static double plan_cost(int M, int N, int K, int bn, int splits, int sms) {
   const long long tiles = tm * tn * s;
   const long long waves = (tiles + sms - 1) / sms;
   const double load = tiles >= sms ? 1.0 : (double)tiles / sms;
-  const double c_kb = 1.0 + 0.7 * load * (128.0 + bn) / 384.0;
-  double cost = waves * (double)(kb_per > 3 ? kb_per : 3) * c_kb + 3.0 * bn / 256.0;
-  if (s > 1) cost += 4.0 + 0.5 * s;
+  const double from_l2 = 0.0070 * load * (kBM + bn) * kBK * 2 / 1024;
+  double cost = fixed + (double)waves * kb_per * (k_block > from_l2 ? k_block : from_l2) + (waves - 1) * 2.0 * bn / 256;
+  if (s > 1) cost += 1.2 + 0.45e-6 * M * N * s;
   return cost;
 }
 
-static int pick_tile_n(int M, int N, int K, int splits) {
-  // 128 x 256 tiles move the fewest operand bytes per FLOP; 192 and 128 win when they fill the last wave better
-  // (widths such as 768 and 3072 = 6 x 128).  A narrower tile must save more than 5% to be taken.
+// `narrow_or_wide`: only the widths 128 and 256 (the weight gather follows its chunks in steps of 128 rows).
+static int pick_tile_n(int M, int N, int K, int splits, bool narrow_or_wide = false) {
   if (N <= 128) return 128;
   const int sms = device_sm_count();
-  const double c256 = plan_cost(M, N, K, 256, splits, sms), c192 = plan_cost(M, N, K, 192, splits, sms),
-               c128 = plan_cost(M, N, K, 128, splits, sms);
-  int bn = 256;
-  double best = c256;
-  if (c192 < best * 0.95) { bn = 192; best = c192; }
-  if (c128 < best * 0.95 && c128 < c256 * 0.95) { bn = 128; best = c128; }
-  return bn;
+  int best_bn = 256;
+  double best = plan_cost(M, N, K, 256, splits, sms);
+  for (int bn : {192, 128}) {
+    if (bn == 192 && narrow_or_wide) continue;
+    const double c = plan_cost(M, N, K, bn, splits, sms);
+    if (c < best) { best = c; best_bn = bn; }
+  }
+  return best_bn;
 }
 
 }  // namespace titb
@@ -1297,7 +1306,7 @@ TITB_API int titb_gemm_pick_splits(int M, int N, int K) {
     for (int bn : {256, 192, 128}) {
       if (bn > 128 && N <= 128) continue;
       const double c = plan_cost(M, N, K, bn, s, sms);
-      if (c < best * (s > best_s ? 0.97 : 1.0)) { best = c; best_s = s; }   // a deeper split must pay for itself
+      if (c < best) { best = c; best_s = s; }
     }
   }
   return best_s;
@@ -1427,12 +1436,13 @@ TITB_API int TITB_GEMM_ENTRY(const TitbGemmDesc* d, cudaStream_t stream) {
   const bool red_split = f32_tma_ok && !deterministic_reductions();
   if (splits > 1 && !red_split && (d->workspace == nullptr || (d->N & 3))) splits = 1;
   // tile_n = 512 asks for CTA pairs on 256 x 256 tiles (cta_group::2); 128 / 192 / 256 are single-CTA 128 x tile_n
-  int bn = d->tile_n ? d->tile_n : pick_tile_n(d->M, d->N, d->K, splits);
-  // CTA pairs for long reductions over an MN-major B operand (weight gradients, and dgrads with a wide output): a pair
-  // stages half of the B tile per CTA.  Measured on the GPT-2 and LLaMA-3 1B layer shapes: up to 16 % faster from 2048
-  // reduction elements per split on, slower below that and on 768-wide dgrad outputs.
-  if (d->tile_n == 0 && d->b_mn_major && (d->coll == nullptr || d->coll->mode == 0) && d->M >= 2 * kBM && d->N >= 256 &&
-      (num_kb + splits - 1) / splits >= 32 && (d->a_mn_major || d->N >= 1024))
+  int bn = d->tile_n ? d->tile_n : pick_tile_n(d->M, d->N, d->K, splits, d->coll != nullptr && d->coll->mode == 3);
+  // CTA pairs stage half of the B tile per CTA, but a k-block of a pair takes 0.345 us against 0.325 of a 128 x 256 tile,
+  // and few tiles leave more of the machine idle.  Where they were faster every time they were measured is tall weight
+  // gradients of four rounds of pairs or more: 50304 x 768 over 2331 tokens 155-161 us against 170-173, 28672 x 4096 over
+  // 4096 799-826 against 850-942; 4096 x 14336 over 4096, wide instead of tall, 347-404 against 339-381.
+  if (d->tile_n == 0 && splits == 1 && d->a_mn_major && d->b_mn_major && (d->coll == nullptr || d->coll->mode == 0) &&
+      d->N >= 256 && d->M >= 4LL * d->N && (d->M / 256LL) * (d->N / 256LL) >= 2LL * device_sm_count())
     bn = 512;
   bool pair = false;
   if (bn == 512) {
@@ -1530,15 +1540,15 @@ TITB_API int TITB_GEMM_ENTRY(const TitbGemmDesc* d, cudaStream_t stream) {
                           (!d->aux_out || (!(reinterpret_cast<uintptr_t>(d->aux_out) & 15) && !(d->ld_aux_out & 7))) &&
                           (!d->aux_in || a.vec_ok) && (!d->bias || a.vec_ok) && g_no_tma_store == 0;
   if (out_tma_ok) {
-    bool okm = make_tmap_bf16_2d(&tout, d->out, d->N, d->M, d->ldo, 64, kBM);
-    if (okm && d->aux_out) okm = make_tmap_bf16_2d(&taux, d->aux_out, d->N, d->M, d->ld_aux_out, 64, kBM);
+    bool okm = make_tmap_bf16_2d(&tout, d->out, d->N, d->M, d->ldo, 64, 32);
+    if (okm && d->aux_out) okm = make_tmap_bf16_2d(&taux, d->aux_out, d->N, d->M, d->ld_aux_out, 64, 32);
     a.tma_store = okm ? 1 : 0;
     if (okm && !d->aux_out && d->aux_in && (d->epilogue == TITB_EPI_DGELU || d->epilogue == TITB_EPI_BIAS_RESIDUAL) &&
         !(reinterpret_cast<uintptr_t>(d->aux_in) & 15) && !(d->ld_aux_in & 7))
-      a.aux_tma_load = make_tmap_bf16_2d(&taux, d->aux_in, d->N, d->M, d->ld_aux_in, 64, kBM) ? 1 : 0;
+      a.aux_tma_load = make_tmap_bf16_2d(&taux, d->aux_in, d->N, d->M, d->ld_aux_in, 64, 32) ? 1 : 0;
   }
   if (f32_tma_ok && (splits == 1 || red_split)) {
-    if (make_tmap_f32_2d(&tout, d->out, d->N, d->M, d->ldo, 32, kBM)) {
+    if (make_tmap_f32_2d(&tout, d->out, d->N, d->M, d->ldo, 32, 32)) {
       a.tma_store = 2;
       a.f32_red = (splits > 1 || d->accumulate) ? 1 : 0;
       if (splits > 1 && !d->accumulate) {   // the partial tiles are added to zeros
