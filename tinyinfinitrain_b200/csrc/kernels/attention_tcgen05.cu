@@ -150,6 +150,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
   __syncthreads();
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  dependency_wait();
+  dependents_launch();
   const uint32_t tS = tmem_base, tO = tmem_base + 128;
   const bool bad_align = (*abort_flag != 0);
 
@@ -485,6 +487,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
   __syncthreads();
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  dependency_wait();
+  dependents_launch();
   const bool bad_align = (*abort_flag != 0);
 
   if (bad_align) {
@@ -807,6 +811,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
 template <int HD>
 __global__ void attn_delta_kernel(const bf16* __restrict__ d_o, const bf16* __restrict__ o, float* __restrict__ delta,
                                   float* __restrict__ dq_accum, int B, int T, int H, long long do_stride_t, long long o_stride_t) {
+  dependents_launch();
   constexpr int L = HD / 8;
   const long long n = static_cast<long long>(B) * T * H * L;
   const long long n_up = (n + 31) / 32 * 32;   // whole warps take part in the shuffles
@@ -838,6 +843,7 @@ __global__ void attn_delta_kernel(const bf16* __restrict__ d_o, const bf16* __re
 // dq (bf16, token stride dq_stride_t) = dq_accum (fp32 [B*T, H*hd])
 __global__ void attn_dq_convert_kernel(const float* __restrict__ acc, bf16* __restrict__ dq, long long BT, int width,
                                        long long dq_stride_t) {
+  dependents_launch();
   const int wv = width / 8;
   const long long n = BT * wv;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -885,7 +891,7 @@ static int attn_fwd_launch(const TitbAttnDesc* d, cudaStream_t st) {
   a.o = static_cast<bf16*>(d->o); a.lse = d->lse; a.o_stride_t = d->o_stride_t;
   a.status = titb_status_ptr();
   dim3 grid((d->T + kBlk - 1) / kBlk, d->Hq, d->B);
-  attn_fwd_kernel<HD><<<grid, kAttnThreads, Cfg::kSmem, st>>>(tq, tk, tv, a);
+  launch_dependent(attn_fwd_kernel<HD>, grid, kAttnThreads, Cfg::kSmem, st, tq, tk, tv, a);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -922,7 +928,7 @@ static int attn_bwd_launch(const TitbAttnDesc* d, cudaStream_t st) {
   a.dk_stride_t = d->dk_stride_t; a.dv_stride_t = d->dv_stride_t;
   a.status = titb_status_ptr();
   dim3 grid(static_cast<unsigned>(d->Hkv) * d->B, (d->T + kBlk - 1) / kBlk);
-  attn_bwd_kernel<HD><<<grid, kBwdThreads, Cfg::kSmem, st>>>(tq, tk, tv, tdo, tdq, a);
+  launch_dependent(attn_bwd_kernel<HD>, grid, kBwdThreads, Cfg::kSmem, st, tq, tk, tv, tdo, tdq, a);
   const long long bt = static_cast<long long>(d->B) * d->T;
   const int width = d->Hq * HD;
   int cb = static_cast<int>((bt * (width / 8) + 255) / 256);

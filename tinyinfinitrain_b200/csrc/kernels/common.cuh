@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <utility>
+
 namespace titb {
 
 using bf16 = __nv_bfloat16;
@@ -113,6 +115,35 @@ __device__ __forceinline__ float gelu_tanh_grad(float x) {
   float t = tanhf(u);
   float du = k * (1.f + 3.f * 0.044715f * x2);
   return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * du;
+}
+
+// Programmatic dependent launch.  A kernel that launch_dependent() starts may become resident while the kernel before it in
+// the stream still drains: its launch, barrier set-up and tensor memory allocation overlap that tail.  It must call
+// dependency_wait() in every thread before the first access to memory that another kernel touches (reads AND writes); the
+// wait ends when the kernel before it has completed and its writes are visible, and because that kernel has waited in its
+// turn, or was launched in the ordinary way, everything before it has, too.  dependents_launch() allows the next kernel of
+// the stream to become resident; it comes after a CTA's own tensor memory allocation, so that the next kernel's CTAs cannot
+// get in front of it.  Both do nothing in an ordinary launch.
+// Launched this way: kernels with one CTA per SM (GEMM, attention backward), with many waves, or tiny ones.  Not kernels whose
+// grid is a few CTAs per SM (column sums, norm backward, element-wise passes): the first SMs to have room would take them
+// all (with them, a LLaMA-3 1B step of 4 x 2048 tokens took 77.8 ms instead of 76.3).  Nor kernels that wait for another GPU.
+// Measured (B200, captured GPT-2 124M steps): 2 x 128 tokens 3.32 -> 3.06-3.11 ms, 3 x 777 5.20 -> 5.02 ms.
+__device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... A>
+inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
 inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }

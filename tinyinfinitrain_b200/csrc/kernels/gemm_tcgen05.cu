@@ -756,6 +756,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
   if (PAIR) ptx::cluster_sync_all();   // the peer's barriers are initialised before anything signals them
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  if (p.coll.mode == 0) dependency_wait();
 
   const int tiles_m = (p.M + kTileM - 1) / kTileM;
   const int tiles_n = (p.N + BN - 1) / BN;
@@ -894,6 +895,11 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
           else ptx::tc_commit(&acc_full[buf]);
         }
       }
+      // The next kernel may come in under the last epilogue.  Not earlier: CTAs that find room on a few SMs only, while the
+      // others still compute, leave the work of a kernel that is one wave wide unevenly spread.
+      if (p.coll.mode == 0) dependents_launch();
+    } else if (PAIR && pair_rank != 0 && lane == 0) {
+      dependents_launch();   // the other CTA of the pair decides
     }
   } else {
     // ---------------------------------------------------------------- epilogue
@@ -1111,6 +1117,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
 template <typename OutT>
 __global__ void splitk_reduce_kernel(const float* __restrict__ ws, OutT* __restrict__ out, long long M, int N,
                                      long long ldo, int splits, int accumulate, const float* __restrict__ alpha) {
+  dependents_launch();
   const long long total = M * N;
   const float al = alpha ? *alpha : 1.f;
   for (long long i = (blockIdx.x * (long long)blockDim.x + threadIdx.x) * 4; i < total;
@@ -1369,13 +1376,15 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
     cfg.blockDim = dim3(kGemmThreads);
     cfg.dynamicSmemBytes = Cfg::kSmem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<BN, PAIR>, ta, tb, tout, taux, args);
     return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
   }
@@ -1409,8 +1418,13 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
     return static_cast<int>(cudaGetLastError());
   }
   int grid = tiles < sms ? tiles : sms;
-  gemm_bf16_tcgen05_kernel<BN, PAIR><<<grid, kGemmThreads, Cfg::kSmem, stream>>>(ta, tb, tout, taux, args);
-  return static_cast<int>(cudaGetLastError());
+  if (args.coll.mode) {
+    gemm_bf16_tcgen05_kernel<BN, PAIR><<<grid, kGemmThreads, Cfg::kSmem, stream>>>(ta, tb, tout, taux, args);
+    return static_cast<int>(cudaGetLastError());
+  }
+  const cudaError_t e = launch_dependent(gemm_bf16_tcgen05_kernel<BN, PAIR>, grid, kGemmThreads, Cfg::kSmem, stream, ta, tb, tout,
+                                         taux, args);
+  return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }
 
 #ifndef TITB_GEMM_PARAM_GATHER

@@ -36,6 +36,8 @@ template <typename T, int MAXV, int G, bool RMS>
 __global__ void norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ b,
                                 T* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out,
                                 long long rows, int C, float eps) {
+  dependency_wait();
+  dependents_launch();
   constexpr int VN = VecN<T>::n;
   __shared__ float red[2 * (G > 32 ? G / 32 : 1)];
   const int tig = (G == 32) ? (threadIdx.x & 31) : threadIdx.x;  // thread in group
@@ -102,6 +104,7 @@ __global__ void norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ 
                                 const T* __restrict__ dres, const float* __restrict__ mean_in,
                                 const float* __restrict__ rstd_in, T* __restrict__ dx, float* __restrict__ scratch,
                                 long long rows, int C, int nparts) {
+  dependents_launch();
   constexpr int VN = VecN<T>::n;
   __shared__ float red[2 * (G > 32 ? G / 32 : 1)];
   const int tig = (G == 32) ? (threadIdx.x & 31) : threadIdx.x;
@@ -239,6 +242,7 @@ __global__ void __launch_bounds__(256, 2)
 norm_bwd_rows2_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ w,
                       const T* __restrict__ dres, const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
                       T* __restrict__ dx, float* __restrict__ scratch, long long rows, int C, int nparts) {
+  dependents_launch();
   constexpr int VN = VecN<T>::n;
   constexpr int Q = VN / 4;                       // float4 groups per 128-bit vector
   constexpr int kPerWarp = NV * Q * 32 * 4;       // floats of one gradient held by one warp
@@ -412,6 +416,8 @@ __device__ __forceinline__ void fold_partial_rows(const float* __restrict__ src,
 __global__ void __launch_bounds__(32 * kFoldTy)
 partial_colsum2_kernel(const float* __restrict__ scratch, float* __restrict__ dw, float* __restrict__ db, int used,
                        int nparts, int C, int accumulate) {
+  dependency_wait();
+  dependents_launch();
   fold_partial_rows(scratch + (long long)blockIdx.y * nparts * C, blockIdx.y == 0 ? dw : db, used, C, accumulate);
 }
 
@@ -508,11 +514,11 @@ static int norm_fwd_launch(const void* x, const void* w, const void* b, void* y,
   const bool aligned = !((uintptr_t)x & 15) && !((uintptr_t)y & 15) && !((uintptr_t)w & 15) && !((uintptr_t)b & 15);
   if (p.G == 32 && aligned) {
     const int blocks = (int)((rows + 3) / 4);
-    if (p.maxv == 4) norm_fwd_kernel<T, 4, 32, RMS><<<blocks, 128, 0, st>>>(X, W, Bv, Y, mean, rstd, rows, C, eps);
-    else norm_fwd_kernel<T, 8, 32, RMS><<<blocks, 128, 0, st>>>(X, W, Bv, Y, mean, rstd, rows, C, eps);
+    if (p.maxv == 4) launch_dependent(norm_fwd_kernel<T, 4, 32, RMS>, blocks, 128, 0, st, X, W, Bv, Y, mean, rstd, rows, C, eps);
+    else launch_dependent(norm_fwd_kernel<T, 8, 32, RMS>, blocks, 128, 0, st, X, W, Bv, Y, mean, rstd, rows, C, eps);
   } else if (p.G == 256 && aligned) {
-    if (p.maxv == 2) norm_fwd_kernel<T, 2, 256, RMS><<<(unsigned)rows, 256, 0, st>>>(X, W, Bv, Y, mean, rstd, rows, C, eps);
-    else norm_fwd_kernel<T, 8, 256, RMS><<<(unsigned)rows, 256, 0, st>>>(X, W, Bv, Y, mean, rstd, rows, C, eps);
+    if (p.maxv == 2) launch_dependent(norm_fwd_kernel<T, 2, 256, RMS>, (unsigned)rows, 256, 0, st, X, W, Bv, Y, mean, rstd, rows, C, eps);
+    else launch_dependent(norm_fwd_kernel<T, 8, 256, RMS>, (unsigned)rows, 256, 0, st, X, W, Bv, Y, mean, rstd, rows, C, eps);
   } else {
     norm_fwd_generic<T, RMS><<<(unsigned)rows, 256, 0, st>>>(X, W, Bv, Y, mean, rstd, rows, C, eps);
   }
@@ -556,7 +562,7 @@ static int norm_bwd_launch(const void* dy, const void* x, const void* w, const v
       if (p.maxv == 2) norm_bwd_kernel<T, 2, 256, RMS><<<used, 256, 0, st>>>(DY, X, W, R, mean, rstd, DX, scratch, rows, C, nparts);
       else norm_bwd_kernel<T, 8, 256, RMS><<<used, 256, 0, st>>>(DY, X, W, R, mean, rstd, DX, scratch, rows, C, nparts);
     }
-    partial_colsum2_kernel<<<dim3((C + 31) / 32, (!RMS && db) ? 2 : 1), 32 * kFoldTy, 0, st>>>(scratch, dw, db, used, nparts, C, accumulate);
+    launch_dependent(partial_colsum2_kernel, dim3((C + 31) / 32, (!RMS && db) ? 2 : 1), 32 * kFoldTy, 0, st, scratch, dw, db, used, nparts, C, accumulate);
   } else {
     norm_bwd_dx_generic<T, RMS><<<(unsigned)rows, 256, 0, st>>>(DY, X, W, R, mean, rstd, DX, rows, C);
     norm_bwd_dw_generic<T, RMS><<<(C + 127) / 128, 128, 0, st>>>(DY, X, mean, rstd, dw, db, rows, C, accumulate);

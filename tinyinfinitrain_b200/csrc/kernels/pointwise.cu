@@ -73,6 +73,7 @@ __device__ __forceinline__ float sigmoidf_(float x) { return 1.f / (1.f + __expf
 // SwiGLU over a fused [rows, 2F] projection.
 template <typename T>
 __global__ void swiglu_fwd_kernel(const T* __restrict__ x, T* __restrict__ y, long long rows, int F) {
+  dependents_launch();
   constexpr int VN = VecN<T>::n;
   const int fv = F / VN;
   const long long total = rows * fv;
@@ -91,6 +92,7 @@ __global__ void swiglu_fwd_kernel(const T* __restrict__ x, T* __restrict__ y, lo
 template <typename T>
 __global__ void swiglu_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, T* __restrict__ dx, long long rows,
                                   int F) {
+  dependents_launch();
   constexpr int VN = VecN<T>::n;
   const int fv = F / VN;
   const long long total = rows * fv;
@@ -115,6 +117,7 @@ __global__ void swiglu_bwd_kernel(const T* __restrict__ dy, const T* __restrict_
 template <typename T>
 __global__ void rope_kernel(const T* x, T* y, long long BT, int T_, int H, int hd, long long stride_t,
                             int pos_offset, float log2_theta, int inverse) {
+  dependents_launch();
   constexpr int VN = VecN<T>::n;
   const int half = hd / 2;
   const int hv = half / VN;
@@ -223,6 +226,7 @@ constexpr int kColsumParts = 296;  // partial rows in the caller-provided scratc
 template <typename T, int NV>
 __global__ void __launch_bounds__(256, 2) colsum_rows_kernel(const T* __restrict__ x, float* __restrict__ scratch,
                                                           long long rows, int C) {
+  dependents_launch();
   constexpr int VN = VecN<T>::n;
   constexpr int kStrip = 32 * NV * VN;
   __shared__ float sm[kStrip];
@@ -282,6 +286,8 @@ __global__ void __launch_bounds__(256, 2) colsum_rows_kernel(const T* __restrict
 constexpr int kFoldTy = 32;
 __global__ void __launch_bounds__(32 * kFoldTy)
 colsum_stage2(const float* __restrict__ scratch, float* __restrict__ out, int nparts, int C, int accumulate) {
+  dependency_wait();
+  dependents_launch();
   __shared__ float sm[kFoldTy][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + tx;
@@ -477,7 +483,7 @@ TITB_API int titb_colsum(const void* x, float* out, long long rows, int C, int d
       if (nv == 3) colsum_rows_kernel<float, 3><<<grid, 256, 0, st>>>((const float*)x, scratch, rows, C);
       else colsum_rows_kernel<float, 4><<<grid, 256, 0, st>>>((const float*)x, scratch, rows, C);
     }
-    colsum_stage2<<<(C + 31) / 32, 32 * kFoldTy, 0, st>>>(scratch, out, parts, C, accumulate);
+    launch_dependent(colsum_stage2, (C + 31) / 32, 32 * kFoldTy, 0, st, scratch, out, parts, C, accumulate);
   } else {
     if (dtype == 1) colsum_generic<bf16><<<(C + 127) / 128, 128, 0, st>>>((const bf16*)x, out, rows, C, accumulate);
     else colsum_generic<float><<<(C + 127) / 128, 128, 0, st>>>((const float*)x, out, rows, C, accumulate);

@@ -137,6 +137,8 @@ __global__ void __launch_bounds__(kSThreads, 1) sgemm_split3_kernel(const SgemmA
   __syncthreads();
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  dependency_wait();
+  dependents_launch();
 
   const int tiles_m = (p.M + kST - 1) / kST, tiles_n = (p.N + kST - 1) / kST;
   const int tiles = tiles_m * tiles_n;
@@ -382,13 +384,15 @@ TITB_API int titb_sgemm(const float* A, const float* B, float* C, int M, int N, 
   cfg.blockDim = dim3(kSThreads);
   cfg.dynamicSmemBytes = kSSmem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = a.split;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   cudaError_t e = cudaLaunchKernelEx(&cfg, sgemm_split3_kernel, a);
   return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }

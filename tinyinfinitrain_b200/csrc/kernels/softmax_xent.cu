@@ -42,6 +42,8 @@ template <typename T>
 __global__ void __launch_bounds__(512)
 xent_kernel(const T* logits, const long long* __restrict__ targets, float* __restrict__ losses,
             T* dlogits, int V, long long ld, float grad_scale, const float* __restrict__ upstream, int vec_ok) {
+  dependency_wait();
+  dependents_launch();
   constexpr int VN = VecN<T>::n;
   __shared__ float red[64];
   const long long row = blockIdx.x;
@@ -237,9 +239,9 @@ TITB_API int titb_xent_fwd_bwd(const void* logits, const long long* targets, flo
   const int vec_ok = !((uintptr_t)logits & 15) && !((uintptr_t)dlogits & 15) && (ld % vn == 0);
   const int threads = V >= 8192 ? 512 : 128;
   if (dtype == 1)
-    xent_kernel<bf16><<<(unsigned)rows, threads, 0, st>>>((const bf16*)logits, targets, losses, (bf16*)dlogits, V, ld, grad_scale, nullptr, vec_ok);
+    launch_dependent(xent_kernel<bf16>, (unsigned)rows, threads, 0, st, (const bf16*)logits, targets, losses, (bf16*)dlogits, V, ld, grad_scale, nullptr, vec_ok);
   else
-    xent_kernel<float><<<(unsigned)rows, threads, 0, st>>>((const float*)logits, targets, losses, (float*)dlogits, V, ld, grad_scale, nullptr, vec_ok);
+    launch_dependent(xent_kernel<float>, (unsigned)rows, threads, 0, st, (const float*)logits, targets, losses, (float*)dlogits, V, ld, grad_scale, nullptr, vec_ok);
   return (int)cudaGetLastError();
 }
 
@@ -251,9 +253,9 @@ TITB_API int titb_xent_bwd(const void* logits, const long long* targets, void* d
   const int vec_ok = !((uintptr_t)logits & 15) && !((uintptr_t)dlogits & 15) && (ld % vn == 0);
   const int threads = V >= 8192 ? 512 : 128;
   if (dtype == 1)
-    xent_kernel<bf16><<<(unsigned)rows, threads, 0, st>>>((const bf16*)logits, targets, nullptr, (bf16*)dlogits, V, ld, grad_scale, upstream, vec_ok);
+    launch_dependent(xent_kernel<bf16>, (unsigned)rows, threads, 0, st, (const bf16*)logits, targets, nullptr, (bf16*)dlogits, V, ld, grad_scale, upstream, vec_ok);
   else
-    xent_kernel<float><<<(unsigned)rows, threads, 0, st>>>((const float*)logits, targets, nullptr, (float*)dlogits, V, ld, grad_scale, upstream, vec_ok);
+    launch_dependent(xent_kernel<float>, (unsigned)rows, threads, 0, st, (const float*)logits, targets, nullptr, (float*)dlogits, V, ld, grad_scale, upstream, vec_ok);
   return (int)cudaGetLastError();
 }
 
