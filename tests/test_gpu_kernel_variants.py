@@ -232,6 +232,46 @@ def test_attention_pipelines_forward_and_backward(B, T, Hq, Hkv, hd):
     assert torch.equal(grads[0][..., kv], grads[1][..., kv])
 
 
+@pytest.mark.parametrize("rows", [1, 2, 1185])
+@pytest.mark.parametrize("dtype,cols", [(BF, 1032), (BF, 2048), (BF, 2056), (BF, 4096), (BF, 4104), (torch.float32, 516), (torch.float32, 2048)])
+@pytest.mark.parametrize("rms", [False, True])
+def test_norm_backward_at_the_edges_of_its_kernels(dtype, cols, rows, rms):
+    """129, 256, 257, 512 and 513 vectors per row; a single row, one pair, and one row more than the CTAs take in one go.
+    Against float64 on the same inputs and statistics: dx is one rounding of its type away from fp32 sums over the row, the
+    weight gradients are fp32 sums over the rows (errors below 2^-24 per addition of the magnitudes)."""
+    torch.manual_seed(37)
+    x, dy, res = (torch.randn(rows, cols, device=DEV).to(dtype) for _ in range(3))
+    w, b = (torch.rand(cols, device=DEV) + 0.5).to(dtype), torch.zeros(cols, device=DEV, dtype=dtype)
+    if rms:
+        rstd = C.rmsnorm_fwd(x, w, 1e-5)[1]
+        mean = torch.zeros_like(rstd)
+        dx, dw = C.rmsnorm_bwd(dy, x, w, rstd, dres=res)
+    else:
+        _, mean, rstd = C.layernorm_fwd(x, w, b, 1e-5)
+        dx, dw, db = C.layernorm_bwd(dy, x, w, mean, rstd, dres=res)
+    r = rstd.double().view(-1, 1)
+    n = (x.double() - mean.double().view(-1, 1)) * r
+    dn = dy.double() * w.double()
+    m1 = 0.0 if rms else dn.mean(1, keepdim=True)
+    ref = (dn - m1 - n * (dn * n).mean(1, keepdim=True)) * r + res.double()
+    eps = 2.0 ** -8 if dtype == BF else 2.0 ** -20
+    assert ((dx.double() - ref).abs() <= eps * ref.abs() + 2e-5).all()
+    bound = 2.0 ** -8 if dw.dtype == BF else (rows + 8) * 2.0 ** -23
+    assert ((dw.double() - (dy.double() * n).sum(0)).abs() <= bound * (dy.double() * n).abs().sum(0) + 1e-6).all()
+    if not rms:
+        assert ((db.double() - dy.double().sum(0)).abs() <= bound * dy.double().abs().sum(0) + 1e-6).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, BF])
+@pytest.mark.parametrize("rows,cols", [(1, 8), (9, 1032), (25, 3080), (2400, 776), (4737, 1600)])
+def test_column_sums_of_ragged_strips(dtype, rows, cols):
+    """Strips that end inside a warp, and warps with none, one or a few rows: every float against float64, fp32 sums."""
+    torch.manual_seed(41)
+    x = torch.randn(rows, cols, device=DEV).to(dtype)
+    out = C.colsum(x, None, False).double()
+    assert ((out - x.double().sum(0)).abs() <= (rows + 8) * 2.0 ** -24 * x.double().abs().sum(0)).all()
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, BF])
 @pytest.mark.parametrize("rows,cols", [(8192, 768), (8192, 3072), (1000, 2304), (37, 264), (5, 8), (4099, 1000)])
 def test_column_sums_in_fixed_order(dtype, rows, cols):

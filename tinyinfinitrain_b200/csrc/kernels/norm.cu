@@ -97,8 +97,8 @@ __global__ void norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ w
   }
 }
 
-// Backward.  Every group walks rows with a grid stride and keeps dw/db partial sums
-// for the columns it owns in registers; the partials go to scratch[2][nparts][C].
+// Backward for very wide rows (more than 512 vectors): a CTA of G threads owns a row, walks rows with a grid stride and
+// keeps the dw/db partial sums of its columns in registers; the partials go to scratch[2][nparts][C].
 template <typename T, int MAXV, int G, bool RMS>
 __global__ void norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ w,
                                 const T* __restrict__ dres, const float* __restrict__ mean_in,
@@ -106,12 +106,8 @@ __global__ void norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ 
                                 long long rows, int C, int nparts) {
   dependents_launch();
   constexpr int VN = VecN<T>::n;
-  __shared__ float red[2 * (G > 32 ? G / 32 : 1)];
-  const int tig = (G == 32) ? (threadIdx.x & 31) : threadIdx.x;
-  const int groups_per_block = (G == 32) ? (blockDim.x >> 5) : 1;
-  const int gib = (G == 32) ? (threadIdx.x >> 5) : 0;  // group in block
-  const long long group = blockIdx.x * (long long)groups_per_block + gib;
-  const long long ngroups = gridDim.x * (long long)groups_per_block;
+  __shared__ float red[2 * (G / 32)];
+  const int tig = threadIdx.x;
   const int nvec = C / VN;
 
   float dwacc[MAXV][VN], dbacc[MAXV][VN];
@@ -124,7 +120,7 @@ __global__ void norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ 
     if (i < nvec) wv[k] = ld128(w + i * VN);
   }
 
-  for (long long row = group; row < rows; row += ngroups) {
+  for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
     const float mean = RMS ? 0.f : mean_in[row];
     const float rstd = rstd_in[row];
     const T* xr = x + row * C;
@@ -171,43 +167,16 @@ __global__ void norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ 
     }
   }
 
-  // Stage 1 of the dw/db reduction: the groups of a CTA fold their sums in a fixed
-  // order through shared memory, then the CTA writes one partial row.
-  extern __shared__ float acc_smem[];  // [2][C] when G == 32
   float* dwp = scratch + (long long)blockIdx.x * C;
   float* dbp = scratch + ((long long)nparts + blockIdx.x) * C;
-  if constexpr (G == 32) {
-    for (int g = 0; g < groups_per_block; ++g) {
-      if (gib == g) {
 #pragma unroll
-        for (int k = 0; k < MAXV; ++k) {
-          const int i = tig + k * G;
-          if (i < nvec) {
+  for (int k = 0; k < MAXV; ++k) {
+    const int i = tig + k * G;
+    if (i < nvec) {
 #pragma unroll
-            for (int e = 0; e < VN; ++e) {
-              const int c = i * VN + e;
-              acc_smem[c] = (g == 0 ? 0.f : acc_smem[c]) + dwacc[k][e];
-              if (!RMS) acc_smem[C + c] = (g == 0 ? 0.f : acc_smem[C + c]) + dbacc[k][e];
-            }
-          }
-        }
-      }
-      __syncthreads();
-    }
-    for (int c = threadIdx.x; c < C; c += blockDim.x) {
-      dwp[c] = acc_smem[c];
-      if (!RMS) dbp[c] = acc_smem[C + c];
-    }
-  } else {
-#pragma unroll
-    for (int k = 0; k < MAXV; ++k) {
-      const int i = tig + k * G;
-      if (i < nvec) {
-#pragma unroll
-        for (int e = 0; e < VN; ++e) {
-          dwp[i * VN + e] = dwacc[k][e];
-          if (!RMS) dbp[i * VN + e] = dbacc[k][e];
-        }
+      for (int e = 0; e < VN; ++e) {
+        dwp[i * VN + e] = dwacc[k][e];
+        if (!RMS) dbp[i * VN + e] = dbacc[k][e];
       }
     }
   }
@@ -382,6 +351,138 @@ norm_bwd_rows2_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T
   }
 }
 
+// Backward for rows of 129 to 512 vectors (bf16: widths 1032 to 4096).  A warp that held such a row alone kept 64 or more
+// sums per thread and had eight rows a SM in flight, a quarter of what hides the memory latency.  Here 256 threads share
+// a row, NV vectors each, and two rows are in flight per CTA, MINB CTAs per SM; the four row sums of the pair take one barrier
+// (the scratch for them alternates).  dweight / dbias sums stay in registers, one partial row per CTA at the end.
+// Bound: memory, three (with a residual gradient four) passes of rows x C.  Measured with the fold of the partial rows (B200,
+// residual gradient; before = a warp per row, 4096: a row per CTA): 8192 x 2048 RMS 97.9 -> 33.9 us, 4096 x 1600 53.0 -> 21.0 us,
+// 4096 x 4096 RMS 60.1 -> 37.9 us, fp32 128 x 768 12.9 -> 4.3 us.
+template <typename T, int NV, bool RMS, int MINB>
+__global__ void __launch_bounds__(256, MINB)
+norm_bwd_cta_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ dres,
+                    const float* __restrict__ mean_in, const float* __restrict__ rstd_in, T* __restrict__ dx,
+                    float* __restrict__ scratch, long long rows, int C, int nparts) {
+  dependents_launch();
+  constexpr int VN = VecN<T>::n;
+  __shared__ float4 red[2][8];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int nvec = C / VN;
+  const float invC = 1.f / C;
+
+  float dwacc[NV][VN], dbacc[RMS ? 1 : NV][RMS ? 1 : VN];
+  Pack<T, VN> wv[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const int i = t + k * 256;
+    if (i < nvec) wv[k] = ld128(w + i * VN);
+#pragma unroll
+    for (int e = 0; e < VN; ++e) {
+      dwacc[k][e] = 0.f;
+      if constexpr (!RMS) dbacc[k][e] = 0.f;
+    }
+  }
+
+  int par = 0;
+  for (long long r0 = blockIdx.x; r0 < rows; r0 += 2LL * gridDim.x, par ^= 1) {
+    const long long r1 = r0 + gridDim.x;
+    const bool has1 = r1 < rows;
+    Pack<T, VN> xa[NV], da[NV], xb[NV], db_[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const int i = t + k * 256;
+      if (i < nvec) {
+        xa[k] = ld128(x + r0 * C + i * VN);
+        da[k] = ld128(dy + r0 * C + i * VN);
+        if (has1) {
+          xb[k] = ld128(x + r1 * C + i * VN);
+          db_[k] = ld128(dy + r1 * C + i * VN);
+        }
+      }
+    }
+    const float mean0 = RMS ? 0.f : mean_in[r0], rstd0 = rstd_in[r0];
+    const float mean1 = (RMS || !has1) ? 0.f : mean_in[r1], rstd1 = has1 ? rstd_in[r1] : 0.f;
+    float s1a = 0.f, s2a = 0.f, s1b = 0.f, s2b = 0.f;  // sum(dnorm), sum(dnorm * norm) of the two rows
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      if (t + k * 256 < nvec) {
+#pragma unroll
+        for (int e = 0; e < VN; ++e) {
+          const float wf = to_f32(wv[k].v[e]);
+          const float n0 = (to_f32(xa[k].v[e]) - mean0) * rstd0;
+          const float g0 = to_f32(da[k].v[e]);
+          s1a += g0 * wf;
+          s2a += g0 * wf * n0;
+          dwacc[k][e] += g0 * n0;
+          if constexpr (!RMS) dbacc[k][e] += g0;
+          if (has1) {
+            const float n1 = (to_f32(xb[k].v[e]) - mean1) * rstd1;
+            const float g1 = to_f32(db_[k].v[e]);
+            s1b += g1 * wf;
+            s2b += g1 * wf * n1;
+            dwacc[k][e] += g1 * n1;
+            if constexpr (!RMS) dbacc[k][e] += g1;
+          }
+        }
+      }
+    }
+    warp_sum4(s1a, s2a, s1b, s2b);
+    if (lane == 0) red[par][warp] = make_float4(s1a, s2a, s1b, s2b);
+    __syncthreads();
+    s1a = s2a = s1b = s2b = 0.f;
+#pragma unroll
+    for (int g = 0; g < 8; ++g) {
+      const float4 f = red[par][g];
+      s1a += f.x; s2a += f.y; s1b += f.z; s2b += f.w;
+    }
+    const float m1a = RMS ? 0.f : s1a * invC, m2a = s2a * invC;
+    const float m1b = RMS ? 0.f : s1b * invC, m2b = s2b * invC;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      opaque128(xa[k]); opaque128(da[k]); opaque128(xb[k]); opaque128(db_[k]);   // unpack again (see above)
+      const int i = t + k * 256;
+      if (i < nvec) {
+        Pack<T, VN> oa, ob, ra, rb;
+        if (dres != nullptr) {
+          ra = ld128(dres + r0 * C + i * VN);
+          if (has1) rb = ld128(dres + r1 * C + i * VN);
+        }
+#pragma unroll
+        for (int e = 0; e < VN; ++e) {
+          const float wf = to_f32(wv[k].v[e]);
+          const float n0 = (to_f32(xa[k].v[e]) - mean0) * rstd0;
+          float o0 = (to_f32(da[k].v[e]) * wf - m1a - n0 * m2a) * rstd0;
+          if (dres != nullptr) o0 += to_f32(ra.v[e]);
+          oa.v[e] = from_f32<T>(o0);
+          if (has1) {
+            const float n1 = (to_f32(xb[k].v[e]) - mean1) * rstd1;
+            float o1 = (to_f32(db_[k].v[e]) * wf - m1b - n1 * m2b) * rstd1;
+            if (dres != nullptr) o1 += to_f32(rb.v[e]);
+            ob.v[e] = from_f32<T>(o1);
+          }
+        }
+        st128(dx + r0 * C + i * VN, oa);
+        if (has1) st128(dx + r1 * C + i * VN, ob);
+      }
+    }
+  }
+
+  float* dwp = scratch + (long long)blockIdx.x * C;
+  float* dbp = scratch + ((long long)nparts + blockIdx.x) * C;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const int i = t + k * 256;
+    if (i < nvec) {
+#pragma unroll
+      for (int e = 0; e < VN; e += 4) {
+        *reinterpret_cast<float4*>(dwp + i * VN + e) = make_float4(dwacc[k][e], dwacc[k][e + 1], dwacc[k][e + 2], dwacc[k][e + 3]);
+        if constexpr (!RMS)
+          *reinterpret_cast<float4*>(dbp + i * VN + e) = make_float4(dbacc[k][e], dbacc[k][e + 1], dbacc[k][e + 2], dbacc[k][e + 3]);
+      }
+    }
+  }
+}
+
 // Stage 2: out[c] (+)= sum_p scratch[p][c] in a fixed order.  The partial rows are a megabyte at most, so the pass is
 // pure latency: 32 columns per CTA and kFoldTy threads per column, each summing every kFoldTy-th partial row with four
 // independent accumulators (four loads in flight), then one fixed-order fold through shared memory.
@@ -540,11 +641,12 @@ static int norm_bwd_launch(const void* dy, const void* x, const void* w, const v
                        !((uintptr_t)dres & 15);
   if (p.G != 0 && aligned && scratch != nullptr) {
     const int nparts = kNormBwdParts;  // scratch is [2][kNormBwdParts][C]; the first `used` rows are written
+    const int nvec = C / VN;
     int used;
-    if (p.G == 32) {
+    if (nvec <= 128) {
       used = 2 * device_sm_count();
       if (used > kNormBwdBlocks) used = kNormBwdBlocks;
-      const int nv = (C / VN + 31) / 32;  // 128-bit vectors per lane
+      const int nv = (nvec + 31) / 32;  // 128-bit vectors per lane
       auto launch = [&](auto kern, int NVc) {
         // per warp and gradient: NVc vectors * VN floats * 32 lanes
         const size_t sm = 8 * (size_t)(RMS ? 1 : 2) * NVc * VN * 32 * sizeof(float);
@@ -552,15 +654,19 @@ static int norm_bwd_launch(const void* dy, const void* x, const void* w, const v
         kern<<<used, 256, sm, st>>>(DY, X, W, R, mean, rstd, DX, scratch, rows, C, nparts);
       };
       if (nv <= 3) launch(norm_bwd_rows2_kernel<T, 3, RMS>, 3);
-      else if (nv <= 4) launch(norm_bwd_rows2_kernel<T, 4, RMS>, 4);
-      else {  // up to 8 vectors per lane: one row at a time per warp, sums in registers
-        used = kNormBwdBlocks;
-        norm_bwd_kernel<T, 8, 32, RMS><<<used, 128, 2 * (size_t)C * sizeof(float), st>>>(DY, X, W, R, mean, rstd, DX, scratch, rows, C, nparts);
-      }
+      else launch(norm_bwd_rows2_kernel<T, 4, RMS>, 4);
+    } else if (nvec <= 512 && !((uintptr_t)scratch & 15)) {
+      // a CTA per pair of rows; no more CTAs than pairs, so that a short input leaves few partial rows to fold
+      const bool narrow = nvec <= 256;
+      const long long pairs = (rows + 1) / 2;
+      used = (narrow ? 4 : 2) * device_sm_count();
+      if (used > kNormBwdParts) used = kNormBwdParts;
+      if (used > pairs) used = (int)pairs;
+      if (narrow) norm_bwd_cta_kernel<T, 1, RMS, 4><<<used, 256, 0, st>>>(DY, X, W, R, mean, rstd, DX, scratch, rows, C, nparts);
+      else norm_bwd_cta_kernel<T, 2, RMS, 2><<<used, 256, 0, st>>>(DY, X, W, R, mean, rstd, DX, scratch, rows, C, nparts);
     } else {
       used = kNormBwdParts;
-      if (p.maxv == 2) norm_bwd_kernel<T, 2, 256, RMS><<<used, 256, 0, st>>>(DY, X, W, R, mean, rstd, DX, scratch, rows, C, nparts);
-      else norm_bwd_kernel<T, 8, 256, RMS><<<used, 256, 0, st>>>(DY, X, W, R, mean, rstd, DX, scratch, rows, C, nparts);
+      norm_bwd_kernel<T, 8, 256, RMS><<<used, 256, 0, st>>>(DY, X, W, R, mean, rstd, DX, scratch, rows, C, nparts);
     }
     launch_dependent(partial_colsum2_kernel, dim3((C + 31) / 32, (!RMS && db) ? 2 : 1), 32 * kFoldTy, 0, st, scratch, dw, db, used, nparts, C, accumulate);
   } else {
