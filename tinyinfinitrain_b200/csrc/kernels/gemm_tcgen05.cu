@@ -1237,8 +1237,9 @@ static int g_no_tma_store = 0;  // set by titb_gemm_set_tma_store(0): A/B switch
 //   k-block   how long 64 reduction steps of a tile take: the MMAs, or on a full machine the operand bytes out of L2
 //   fixed     launch, pipeline fill, the last epilogue
 //   epilogue  what the next main loop does not hide of an epilogue
-//   a split   zero fill of the output, and the reduce-adds of the partial tiles
-static double plan_cost(int M, int N, int K, int bn, int splits, int sms) {
+//   a split   zero fill of the output, and the reduce-adds of the partial tiles; or (`workspace`) the partial tiles written,
+//             read and summed by a second kernel, 8 bytes per element and split
+static double plan_cost(int M, int N, int K, int bn, int splits, int sms, bool workspace = false) {
   const double k_block = bn == 128 ? 0.224 : bn == 192 ? 0.241 : 0.325, fixed = bn == 128 ? 5.0 : bn == 192 ? 6.1 : 5.6;
   const long long tm = (M + kBM - 1) / kBM, tn = (N + bn - 1) / bn;
   const int kb = (K + kBK - 1) / kBK;
@@ -1249,7 +1250,7 @@ static double plan_cost(int M, int N, int K, int bn, int splits, int sms) {
   const double load = tiles >= sms ? 1.0 : (double)tiles / sms;
   const double from_l2 = 0.0070 * load * (kBM + bn) * kBK * 2 / 1024;
   double cost = fixed + (double)waves * kb_per * (k_block > from_l2 ? k_block : from_l2) + (waves - 1) * 2.0 * bn / 256;
-  if (s > 1) cost += 1.2 + 0.45e-6 * M * N * s;
+  if (s > 1) cost += workspace ? 4.0 + 1.6e-6 * M * N * s : 1.2 + 0.45e-6 * M * N * s;
   return cost;
 }
 
@@ -1299,7 +1300,7 @@ TITB_API void titb_gemm_set_tma_store(int enabled) { g_no_tma_store = enabled ? 
 
 TITB_API int titb_gemm_pick_tile(int M, int N, int K, int splits) { return pick_tile_n(M, N, K, splits < 1 ? 1 : splits); }
 
-TITB_API int titb_gemm_pick_splits(int M, int N, int K) {
+TITB_API int titb_gemm_pick_splits(int M, int N, int K, int workspace) {
   // Joint choice of split-K factor and tile width by estimated duration (plan_cost): the reduction is split when the
   // output has too few tiles to fill the GPU -- weight gradients: small outputs, K = the token count -- and each
   // split still runs a pipeline of at least 8 k-blocks.  (Callers use the result only where the partial tiles can
@@ -1312,7 +1313,7 @@ TITB_API int titb_gemm_pick_splits(int M, int N, int K) {
     if (s > 1 && kb / s < 8) break;
     for (int bn : {256, 192, 128}) {
       if (bn > 128 && N <= 128) continue;
-      const double c = plan_cost(M, N, K, bn, s, sms);
+      const double c = plan_cost(M, N, K, bn, s, sms, workspace != 0);
       if (c < best) { best = c; best_s = s; }
     }
   }
