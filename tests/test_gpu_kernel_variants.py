@@ -262,6 +262,29 @@ def test_norm_backward_at_the_edges_of_its_kernels(dtype, cols, rows, rms):
         assert ((db.double() - dy.double().sum(0)).abs() <= bound * dy.double().abs().sum(0) + 1e-6).all()
 
 
+@pytest.mark.parametrize("n", [1, 3, 4, 1025, 2047, 2048, 2049, 6145])
+@pytest.mark.parametrize("lp_dtype", [None, torch.float32, BF])
+def test_adam_at_the_edges_of_its_blocks(n, lp_dtype):
+    """Remainders of a vector, of a thread's second vector and of a block; nothing past the end is written.  fp32 arithmetic:
+    a dozen roundings of 2^-24 of the terms; the low-precision copy is one rounding of the result."""
+    torch.manual_seed(43)
+    full = [torch.randn(n + 8, device=DEV), torch.randn(n + 8, device=DEV), torch.randn(n + 8, device=DEV) * 0.1,
+            torch.rand(n + 8, device=DEV) * 0.1]
+    w, g, m, v = (t.double()[:n] for t in full)
+    before = [t.clone() for t in full]
+    lp = torch.zeros(n, device=DEV, dtype=lp_dtype) if lp_dtype is not None else None
+    lr, b1, b2, eps, wd, step = 1e-2, 0.9, 0.95, 1e-8, 0.1, 3
+    C.adam_flat(full[0][:n], lp, full[1][:n], full[2][:n], full[3][:n], lr, b1, b2, eps, wd, step, 0.5, None)
+    m2, v2 = b1 * m + (1 - b1) * 0.5 * g, b2 * v + (1 - b2) * (0.5 * g) ** 2
+    w2 = w - lr * (m2 / (1 - b1 ** step) / ((v2 / (1 - b2 ** step)).sqrt() + eps) + wd * w)
+    for got, want, scale in ((full[2], m2, m.abs() + g.abs()), (full[3], v2, v + g * g), (full[0], w2, w.abs() + lr * 10)):
+        assert ((got[:n].double() - want).abs() <= 2.0 ** -20 * scale).all()
+    for t, old in zip(full, before):
+        assert torch.equal(t[n:], old[n:])
+    if lp is not None:
+        assert torch.equal(lp, full[0][:n].to(lp_dtype))
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, BF])
 @pytest.mark.parametrize("rows,cols", [(1, 8), (9, 1032), (25, 3080), (2400, 776), (4737, 1600)])
 def test_column_sums_of_ragged_strips(dtype, rows, cols):
