@@ -286,6 +286,28 @@ def test_adam_at_the_edges_of_its_blocks(n, lp_dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, BF])
+@pytest.mark.parametrize("B,T,H,hd", [(1, 1, 1, 16), (1, 5, 3, 64), (2, 1024, 40, 64), (1, 1999, 13, 64), (1, 4099, 10, 128)])
+def test_rope_over_groups_of_heads(dtype, B, T, H, hd):
+    """One to eight heads per thread, an odd number of heads, a last group with fewer: both directions against the rotation in
+    float64 at the fp32 angle (which may be a few roundings off: 2^-21 of it), plus one rounding of the type."""
+    torch.manual_seed(47)
+    x = torch.randn(B, T, H, hd, device=DEV).to(dtype)
+    idx = torch.arange(hd // 2, device=DEV, dtype=torch.float64)
+    ang = (torch.arange(T, device=DEV, dtype=torch.float64)[:, None] + 3) * 10000.0 ** (-2 * idx / hd)
+    err = (ang * 2.0 ** -21 + 2.0 ** -22).view(1, T, 1, hd // 2)
+    a, b = x.double().chunk(2, -1)
+    eps = 2.0 ** -8 if dtype == BF else 2.0 ** -22
+    y = ops.rope(x, 3, 10000.0)
+    c, s = ang.cos().view(1, T, 1, -1), ang.sin().view(1, T, 1, -1)
+    for got, want in zip(y.double().chunk(2, -1), (a * c - b * s, b * c + a * s)):
+        assert ((got - want).abs() <= eps * want.abs() + err * (a.abs() + b.abs())).all()
+    xg = x.detach().requires_grad_()
+    ops.rope(xg, 3, 10000.0).backward(x)
+    for got, want in zip(xg.grad.double().chunk(2, -1), (a * c + b * s, b * c - a * s)):
+        assert ((got - want).abs() <= eps * want.abs() + err * (a.abs() + b.abs())).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, BF])
 @pytest.mark.parametrize("rows,cols", [(1, 8), (9, 1032), (25, 3080), (2400, 776), (4737, 1600)])
 def test_column_sums_of_ragged_strips(dtype, rows, cols):
     """Strips that end inside a warp, and warps with none, one or a few rows: every float against float64, fp32 sums."""

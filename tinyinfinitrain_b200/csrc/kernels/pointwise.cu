@@ -113,37 +113,52 @@ __global__ void swiglu_bwd_kernel(const T* __restrict__ dy, const T* __restrict_
   }
 }
 
-// Rotary embedding on [B, T, H, hd]: pairs (i, i + hd/2), angle (t + offset) * theta^(-2i/hd).
+// Rotary embedding on [B, T, H, hd]: pairs (i, i + hd/2), angle (t + offset) * theta^(-2i/hd).  A thread takes VN pairs of one
+// token over up to `per` heads: their angles are the same, and sine and cosine took most of the time when every head
+// computed them (8192 tokens, 40 heads of 64: 28.7 -> 14.5 us).  Two heads are in flight at a time; x and y may be the same.
 template <typename T>
 __global__ void rope_kernel(const T* x, T* y, long long BT, int T_, int H, int hd, long long stride_t,
-                            int pos_offset, float log2_theta, int inverse) {
+                            int pos_offset, float log2_theta, int inverse, int per) {
   dependents_launch();
   constexpr int VN = VecN<T>::n;
   const int half = hd / 2;
   const int hv = half / VN;
-  const long long total = BT * H * hv;
+  const int groups = (H + per - 1) / per;
+  const long long total = BT * groups * hv;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const int v = (int)(i % hv);
-    const long long bth = i / hv;
-    const long long bt = bth / H;
+    const long long btg = i / hv;
+    const long long bt = btg / groups;
     const int t = (int)(bt % T_) + pos_offset;
-    const int hh = (int)(bth - bt * H);
-    const T* xp = x + bt * stride_t + hh * hd + v * VN;
-    T* yp = y + bt * stride_t + hh * hd + v * VN;
-    Pack<T, VN> a = ld128(xp), b = ld128(xp + half), oa, ob;
+    const int h0 = (int)(btg - bt * groups) * per, h1 = min(H, h0 + per);
+    float s[VN], c[VN];
 #pragma unroll
     for (int e = 0; e < VN; ++e) {
       const int idx = v * VN + e;
       const float inv_freq = exp2f(-log2_theta * (2.f * idx / hd));
-      float s, c;
-      sincosf(t * inv_freq, &s, &c);
-      if (inverse) s = -s;
-      const float af = to_f32(a.v[e]), bf = to_f32(b.v[e]);
-      oa.v[e] = from_f32<T>(af * c - bf * s);
-      ob.v[e] = from_f32<T>(bf * c + af * s);
+      sincosf(t * inv_freq, &s[e], &c[e]);
+      if (inverse) s[e] = -s[e];
     }
-    st128(yp, oa);
-    st128(yp + half, ob);
+    for (int h = h0; h < h1; h += 2) {
+      const bool two = h + 1 < h1;
+      const long long off = bt * stride_t + h * hd + v * VN;
+      Pack<T, VN> a[2], b[2];
+      a[0] = ld128(x + off); b[0] = ld128(x + off + half);
+      if (two) { a[1] = ld128(x + off + hd); b[1] = ld128(x + off + hd + half); }
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        if (q == 1 && !two) break;
+        Pack<T, VN> oa, ob;
+#pragma unroll
+        for (int e = 0; e < VN; ++e) {
+          const float af = to_f32(a[q].v[e]), bf = to_f32(b[q].v[e]);
+          oa.v[e] = from_f32<T>(af * c[e] - bf * s[e]);
+          ob.v[e] = from_f32<T>(bf * c[e] + af * s[e]);
+        }
+        st128(y + off + q * hd, oa);
+        st128(y + off + q * hd + half, ob);
+      }
+    }
   }
 }
 
@@ -369,10 +384,15 @@ TITB_API int titb_rope_strided(const void* x, void* y, int B, int T, int H, int 
   if (BT <= 0) return 0;
   const int vn = dtype == 1 ? 8 : 4;
   if ((hd / 2) % vn) return (int)cudaErrorInvalidValue;
-  const int blocks = ew_blocks(BT * H * (hd / 2 / vn));
+  const int hv = hd / 2 / vn;
+  // as many heads per thread as leave every SM 512 threads, 8 at most
+  long long per = BT * H * hv / (device_sm_count() * 512LL);
+  per = per < 1 ? 1 : per > 8 ? 8 : per;
+  if (per > H) per = H;
+  const int blocks = ew_blocks(BT * ((H + per - 1) / per) * hv);
   const float l2 = log2f(theta);
-  if (dtype == 1) rope_kernel<bf16><<<blocks, kEwThreads, 0, st>>>((const bf16*)x, (bf16*)y, BT, T, H, hd, stride_t, pos_offset, l2, inverse);
-  else rope_kernel<float><<<blocks, kEwThreads, 0, st>>>((const float*)x, (float*)y, BT, T, H, hd, stride_t, pos_offset, l2, inverse);
+  if (dtype == 1) rope_kernel<bf16><<<blocks, kEwThreads, 0, st>>>((const bf16*)x, (bf16*)y, BT, T, H, hd, stride_t, pos_offset, l2, inverse, (int)per);
+  else rope_kernel<float><<<blocks, kEwThreads, 0, st>>>((const float*)x, (float*)y, BT, T, H, hd, stride_t, pos_offset, l2, inverse, (int)per);
   return (int)cudaGetLastError();
 }
 
