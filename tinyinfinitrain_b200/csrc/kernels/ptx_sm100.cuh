@@ -81,8 +81,8 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
 }
 
-// The same wait by all 32 lanes of a warp, which leave it together: tcgen05.ld, .st and the cluster barrier must be
-// executed by a converged warp.
+// The same wait by all 32 lanes of a warp, which leave it together and with the same answer: tcgen05.ld and .st must be
+// executed by a converged warp, and a lane that gave up alone would leave the others at their next __syncwarp for good.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
@@ -247,7 +247,10 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-__device__ __forceinline__ void cluster_sync_all() {  // every thread of both CTAs
+// Every thread of every CTA of the cluster.  The instructions are the aligned forms, which a warp must execute converged;
+// callers come from loops and branches that end lane by lane, and a block barrier alone does not bring the lanes together.
+__device__ __forceinline__ void cluster_sync_all() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }

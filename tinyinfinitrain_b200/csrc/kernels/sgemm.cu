@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(kSThreads, 1) sgemm_split3_kernel(const SgemmA
     bool more = tile < tiles && per_tile > 0;
     if (more) load_chunk(tile, c);
     while (more) {
-      if (!ptx::mbar_wait(&empty[stage], phase ^ 1u, abort_flag)) break;
+      if (!ptx::mbar_wait_warp(&empty[stage], phase ^ 1u, abort_flag)) break;
       uint8_t* dst = smem + stage * kSStage;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(kSThreads, 1) sgemm_split3_kernel(const SgemmA
       for (int j = 0; j < 64; ++j) acc[j] = 0.f;
       for (int c = 0; c < per_tile; ++c, ++it) {
         const int buf = it & 1;
-        if (!ptx::mbar_wait(&acc_full[buf], (it >> 1) & 1, abort_flag)) { ok = false; break; }
+        if (!ptx::mbar_wait_warp(&acc_full[buf], (it >> 1) & 1, abort_flag)) { ok = false; break; }
         ptx::tc_fence_after_sync();
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
@@ -290,6 +290,7 @@ __global__ void __launch_bounds__(kSThreads, 1) sgemm_split3_kernel(const SgemmA
   }
 
   ptx::tc_fence_before_sync();
+  __syncwarp();   // the lanes of the MMA warp meet again
   __syncthreads();
   if (p.split > 1) {
     ptx::cluster_sync_all();   // every CTA's partial tile is in its shared memory
