@@ -58,3 +58,84 @@ def test_sgemm_exact_on_small_integers_and_repeatable():
     assert torch.equal(out, (a.double() @ b.double()).float())
     x, y = torch.randn(128, 4096, device=DEV, generator=g), torch.randn(4096, 128, device=DEV, generator=g)
     assert torch.equal(C.sgemm(x, y), C.sgemm(x, y))
+
+
+# ------------------------------------------------------------------ the whole fp32 range
+# one tile, ragged and unaligned, a reduction split over a cluster, several tiles and chunks
+RANGE_SHAPES = [(128, 128, 64), (70, 45, 33), (64, 128, 5000), (130, 260, 192)]
+LAYOUTS = [(False, False), (False, True), (True, False), (True, True)]
+FMAX, INF, NAN = torch.finfo(torch.float32).max, float("inf"), float("nan")
+
+
+def _check(a, b, ta, tb):
+    """Against float64, whose range holds every fp32 product and sum: infinities and NaNs in the same places, the rest within
+    the bound of test_sgemm_against_float64, half of the smallest fp32 number for each rounding, and 2^-148 for each operand
+    below 2^-125: 2^-149 for its third part, twice 2^-150 for the products that are left out (second part at most 2^-134,
+    third at most 2^-142, against 2^-16 and 2^-8 of the other operand)."""
+    A, B = (a.t() if ta else a).double(), (b.t() if tb else b).double()
+    K = A.shape[1]
+    ref, mag = A @ B, A.abs() @ B.abs()
+    out = C.sgemm(a, b, ta, tb)
+    assert C.status_read(True) == 0
+    over = torch.isfinite(ref) & (ref.abs() > FMAX)
+    assert torch.equal(torch.isnan(out), torch.isnan(ref))
+    assert torch.equal(out[torch.isinf(ref)], ref[torch.isinf(ref)].float())
+    fin = torch.isfinite(ref) & ~over
+    small = [(x.abs() < 2.0 ** -125).double() for x in (A, B)]
+    bound = (2 * 5 + (K + 63) // 64 + 2) * 2.0 ** -24 * mag + (K + 1) * 2.0 ** -150
+    bound += 1.01 * 2.0 ** -148 * (small[0] @ B.abs().nan_to_num(posinf=0) + A.abs().nan_to_num(posinf=0) @ small[1])
+    assert bool(((out.double() - ref).abs()[fin] <= bound[fin]).all())
+    start = torch.ones_like(out)
+    C.sgemm(a, b, ta, tb, out=start, accumulate=True)
+    assert torch.equal(start, out + 1) or torch.equal(torch.isnan(start), torch.isnan(out))
+    return out
+
+
+@pytest.mark.parametrize("M,N,K", RANGE_SHAPES)
+@pytest.mark.parametrize("ta,tb", LAYOUTS)
+@pytest.mark.parametrize("value", [-FMAX, FMAX, 3.3961776e38, INF, -INF, NAN])
+def test_sgemm_largest_and_non_finite_operands(M, N, K, ta, tb, value):
+    """One such value in A (a mask's lowest value, say) against small, zero and like values in B."""
+    a, b, A, B = _operands(M, N, K, ta, tb, 3)
+    b.mul_(1e-3)
+    A[5, 7] = value
+    B[7, 3] = 0.0
+    if value in (INF, -INF):
+        B[7, 4] = value
+        B[9, 6] = value
+    out = _check(a, b, ta, tb)
+    assert torch.isfinite(out[:5, :3]).all()
+
+
+@pytest.mark.parametrize("ta,tb", LAYOUTS)
+def test_sgemm_largest_operand_on_the_right(ta, tb):
+    a, b, A, B = _operands(100, 300, 200, ta, tb, 4)
+    a.mul_(1e-3)
+    B[150, 129] = -FMAX
+    B[3, 299] = INF
+    _check(a, b, ta, tb)
+    a.fill_(2.0 ** -100)
+    b.fill_(FMAX)
+    _check(a, b, ta, tb)
+
+
+def test_sgemm_sums_near_the_largest_number():
+    """Parts of a product that are summed apart must not overflow where the sum does not."""
+    a = torch.full((128, 64), 2.0 ** 60, device=DEV)
+    b = torch.full((64, 128), 2.0 ** 61 * (2 - 2.0 ** -23), device=DEV)   # 64 equal terms: the sum is just under 2^128
+    b.mul_(0.99 + 0.01 * torch.rand(64, 128, device=DEV, generator=torch.Generator(device=DEV).manual_seed(5)))
+    out = _check(a, b, False, False)
+    assert torch.isfinite(out).all()
+
+
+@pytest.mark.parametrize("M,N,K", RANGE_SHAPES)
+@pytest.mark.parametrize("ta,tb", [(False, False), (True, True)])
+@pytest.mark.parametrize("exponent", [-100, -110, -115, -120, -126, -135, -149])
+def test_sgemm_small_operands_keep_their_bits(M, N, K, ta, tb, exponent):
+    """Down to the subnormal numbers of A (which hold fewer bits themselves), against ordinary and against large values."""
+    for scale in (1.0, 2.0 ** 100):
+        a, b, A, B = _operands(M, N, K, ta, tb, 6)
+        a.mul_(2.0 ** (exponent / 2)).mul_(2.0 ** (exponent - exponent / 2))
+        b.mul_(scale)
+        _check(a, b, ta, tb)
+        _check(b.t().contiguous(), a.t().contiguous(), tb, ta)   # the small operand on the right

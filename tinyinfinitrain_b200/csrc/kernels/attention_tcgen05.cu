@@ -50,26 +50,6 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
-// two fp32 operations per instruction
-__device__ __forceinline__ void fma2(float& a0, float& a1, float b0, float b1, float c0, float c1, float d0, float d1) {
-  asm("{\n\t.reg .b64 x, y, z;\n\t"
-      "mov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
-      "fma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
-      : "=f"(a0), "=f"(a1) : "f"(b0), "f"(b1), "f"(c0), "f"(c1), "f"(d0), "f"(d1));
-}
-__device__ __forceinline__ void mul2(float& a0, float& a1, float b0, float b1, float c0, float c1) {
-  asm("{\n\t.reg .b64 x, y;\n\t"
-      "mov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
-      "mul.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
-      : "=f"(a0), "=f"(a1) : "f"(b0), "f"(b1), "f"(c0), "f"(c1));
-}
-__device__ __forceinline__ void add2(float& a0, float& a1, float b0, float b1, float c0, float c1) {
-  asm("{\n\t.reg .b64 x, y;\n\t"
-      "mov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
-      "add.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
-      : "=f"(a0), "=f"(a1) : "f"(b0), "f"(b1), "f"(c0), "f"(c1));
-}
-
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float d;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));

@@ -117,6 +117,26 @@ __device__ __forceinline__ float gelu_tanh_grad(float x) {
   return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * du;
 }
 
+// two fp32 operations per instruction
+__device__ __forceinline__ void fma2(float& a0, float& a1, float b0, float b1, float c0, float c1, float d0, float d1) {
+  asm("{\n\t.reg .b64 x, y, z;\n\t"
+      "mov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+      "fma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(a0), "=f"(a1) : "f"(b0), "f"(b1), "f"(c0), "f"(c1), "f"(d0), "f"(d1));
+}
+__device__ __forceinline__ void mul2(float& a0, float& a1, float b0, float b1, float c0, float c1) {
+  asm("{\n\t.reg .b64 x, y;\n\t"
+      "mov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+      "mul.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(a0), "=f"(a1) : "f"(b0), "f"(b1), "f"(c0), "f"(c1));
+}
+__device__ __forceinline__ void add2(float& a0, float& a1, float b0, float b1, float c0, float c1) {
+  asm("{\n\t.reg .b64 x, y;\n\t"
+      "mov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+      "add.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(a0), "=f"(a1) : "f"(b0), "f"(b1), "f"(c0), "f"(c1));
+}
+
 // Programmatic dependent launch.  A kernel that launch_dependent() starts may become resident while the kernel before it in
 // the stream still drains: its launch, barrier set-up and tensor memory allocation overlap that tail.  It must call
 // dependency_wait() in every thread before the first access to memory that another kernel touches (reads AND writes); the

@@ -10,8 +10,15 @@
 // of one fp32 product.  The tensor core truncates when it adds, so it only accumulates over 64 reduction steps, the small
 // products first; those 64-step partial sums are read out of tensor memory and added in registers with round-to-nearest.
 // Against float64 the result is as close as the sequential fp32 FMA chain it replaces, or closer
-// (tests/test_gpu_sgemm.py holds it to that).  Inf and NaN inputs give a non-finite result, not always the same one as IEEE
-// fp32 products (inf - inf appears inside the split).
+// (tests/test_gpu_sgemm.py holds it to that).
+//
+// The range is that of fp32.  x1 and x2 are stored 2^15 times as large, so that they do not fall under the smallest bf16
+// (without it a value below 2^-110 loses bits), and the sum is scaled back by the first MMA of the product that follows.
+// Values below 2^-125 count to within 2^-148, the two last bits of a subnormal number.  At the upper end bf16(x) is infinite
+// from 2^128 (1 - 2^-9) on, inf - inf appears inside the split of an infinity, and scaled parts or products may overflow where
+// x (from 2^120 on) or the sum (from about 2^114 on) does not.  All of these, and NaN operands, leave a non-finite sum: a warp
+// that finds one computes its 32 x 64 piece of the tile again as a chain of fp32 multiply-adds, which gives IEEE's answer
+// (finfo.min as a mask, infinities) at the pace of the CUDA cores, about a sixth of the usual one.
 //
 // Bound: the six products are 6 x 2 M N K tensor FLOPs, i.e. 278 TFLOP/s of fp32 work at the measured bf16 peak, about four
 // times what 148 SMs x 128 FMA lanes can do.  One CTA works on a 128 x 128 tile:
@@ -44,6 +51,8 @@ constexpr int kPlane = kST * kSK * 2;    // one bf16 tile of one operand part: 1
 constexpr int kOperand = 3 * kPlane;
 constexpr int kSStage = 2 * kOperand;    // A and B parts: 96 KB
 constexpr int kSStages = 2;
+constexpr int kPartShift = 15;           // the second and third part of a value are stored 2^15 times as large (the most an MMA scales)
+constexpr float kPartScale = 1 << kPartShift;
 constexpr int kConvWarps = 8, kDrainWarps = 8;
 constexpr int kSThreads = (kConvWarps + kDrainWarps + 1) * 32;
 constexpr int kRedStride = kST + 4;      // floats per row of the partial tile in shared memory (conflict-free 16-byte rows)
@@ -78,16 +87,19 @@ __device__ __forceinline__ void load_unit(float (&v)[8], const float* base, long
   }
 }
 
-// Splits eight values into their three bf16 parts and stores each part's 16 bytes.
+// Splits eight values into their three bf16 parts, the second and the third times kPartScale, and stores each part's 16
+// bytes.  The differences and the scaling are exact.
 __device__ __forceinline__ void split_store(const float (&v)[8], uint8_t* dst) {
   uint32_t p0[4], p1[4], p2[4];
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
-    const float x = v[2 * e], y = v[2 * e + 1];
+    float x = v[2 * e], y = v[2 * e + 1];
     p0[e] = pack_bf16x2(x, y);
-    const float xr = x - __uint_as_float(p0[e] << 16), yr = y - __uint_as_float(p0[e] & 0xffff0000u);
-    p1[e] = pack_bf16x2(xr, yr);
-    p2[e] = pack_bf16x2(xr - __uint_as_float(p1[e] << 16), yr - __uint_as_float(p1[e] & 0xffff0000u));
+    fma2(x, y, __uint_as_float(p0[e] << 16), __uint_as_float(p0[e] & 0xffff0000u), -1.f, -1.f, x, y);
+    mul2(x, y, x, y, kPartScale, kPartScale);
+    p1[e] = pack_bf16x2(x, y);
+    fma2(x, y, __uint_as_float(p1[e] << 16), __uint_as_float(p1[e] & 0xffff0000u), -1.f, -1.f, x, y);
+    p2[e] = pack_bf16x2(x, y);
   }
   *reinterpret_cast<uint4*>(dst) = make_uint4(p0[0], p0[1], p0[2], p0[3]);
   *reinterpret_cast<uint4*>(dst + kPlane) = make_uint4(p1[0], p1[1], p1[2], p1[3]);
@@ -104,6 +116,23 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, uint32_t rank) {
       : "r"(addr), "r"(rank)
       : "memory");
   return v;
+}
+
+// acc[j] = sum over k0 <= k < k1 of op(A)[row, k] op(B)[k, col + j], one rounding per step.  The 32 lanes hold different rows and
+// share the columns, so the loads of B are broadcasts.
+__device__ __forceinline__ void fma_chain(float (&acc)[64], const SgemmArgs& p, int row, int col, int k0, int k1) {
+  const long long a_k = p.a_mn ? p.lda : 1, b_k = p.b_mn ? p.ldb : 1, b_n = p.b_mn ? 1 : p.ldb;
+  const float* a = p.a + (p.a_mn ? row : row * p.lda) + k0 * a_k;
+  const float* b = p.b + col * b_n + k0 * b_k;
+#pragma unroll
+  for (int j = 0; j < 64; ++j) acc[j] = 0.f;
+#pragma unroll 1
+  for (int k = k0; k < k1; ++k, a += a_k, b += b_k) {
+    const float x = __ldg(a);
+#pragma unroll
+    for (int j = 0; j < 64; ++j)
+      if (col + j < p.N) acc[j] = fmaf(x, __ldg(b + j * b_n), acc[j]);
+  }
 }
 
 __global__ void __launch_bounds__(kSThreads, 1) sgemm_split3_kernel(const SgemmArgs p) {
@@ -198,7 +227,8 @@ __global__ void __launch_bounds__(kSThreads, 1) sgemm_split3_kernel(const SgemmA
       const uint32_t idesc = ptx::make_idesc_bf16(kST, kST, p.a_mn, p.b_mn);
       const uint32_t a_lbo = p.a_mn ? 64 * kSK * 2 : 16, b_lbo = p.b_mn ? 64 * kSK * 2 : 16;
       const uint32_t a_step = p.a_mn ? 16 * 128 : 32, b_step = p.b_mn ? 16 * 128 : 32;
-      // smallest products first; {part of A, part of B}
+      // smallest products first; {part of A, part of B}; the first is 2^30 times as large, the last as it is, the
+      // others 2^15 times
       constexpr int kPa[6] = {1, 0, 2, 0, 1, 0}, kPb[6] = {1, 2, 0, 1, 0, 0};
       int stage = 0, it = 0;
       uint32_t phase = 0;
@@ -219,8 +249,11 @@ __global__ void __launch_bounds__(kSThreads, 1) sgemm_split3_kernel(const SgemmA
             const uint64_t ad = ptx::make_smem_desc(sa + kPa[q] * kPlane, a_lbo, 1024);
             const uint64_t bd = ptx::make_smem_desc(sb + kPb[q] * kPlane, b_lbo, 1024);
 #pragma unroll
-            for (int k = 0; k < kSK / 16; ++k)   // only the address field of the descriptors moves
-              ptx::mma_f16_ss(d, ad + ((k * a_step) >> 4), bd + ((k * b_step) >> 4), idesc, (q > 0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < kSK / 16; ++k) {   // only the address field of the descriptors moves
+              const uint64_t ak = ad + ((k * a_step) >> 4), bk = bd + ((k * b_step) >> 4);
+              if (k == 0 && (q == 1 || q == 5)) ptx::mma_f16_ss_scaled<kPartShift>(d, ak, bk, idesc);
+              else ptx::mma_f16_ss(d, ak, bk, idesc, (q > 0 || k > 0) ? 1u : 0u);
+            }
           }
           ptx::tc_commit(&empty[stage]);
           ptx::tc_commit(&acc_full[buf]);
@@ -256,6 +289,12 @@ __global__ void __launch_bounds__(kSThreads, 1) sgemm_split3_kernel(const SgemmA
         if (lane == 0) ptx::mbar_arrive(&acc_empty[buf]);
       }
       if (!ok) break;
+      const int gr = (tile % tiles_m) * kST + row, gc = (tile / tiles_m) * kST + half * 64;
+      float finite = 0.f;
+#pragma unroll
+      for (int j = 0; j < 64; ++j) finite = fmaf(acc[j], 0.f, finite);
+      if (gc < p.N && __any_sync(0xffffffffu, !(finite == 0.f)))
+        fma_chain(acc, p, min(gr, p.M - 1), gc, c0 * kSK, min(p.K, c1 * kSK));
       if (p.split > 1) {
         // every MMA of this CTA has finished (the last accumulator was read), so the operand ring is free
         float* red = reinterpret_cast<float*>(smem) + row * kRedStride + half * 64;
@@ -264,7 +303,6 @@ __global__ void __launch_bounds__(kSThreads, 1) sgemm_split3_kernel(const SgemmA
           *reinterpret_cast<float4*>(red + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
         break;
       }
-      const int gr = (tile % tiles_m) * kST + row, gc = (tile / tiles_m) * kST + half * 64;
       if (gr < p.M && gc < p.N) {
         float* out = p.c + static_cast<long long>(gr) * p.N + gc;
         if (p.c_vec && gc + 64 <= p.N) {
