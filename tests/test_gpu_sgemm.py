@@ -1,4 +1,8 @@
 """fp32 GEMM on the tensor cores (csrc/kernels/sgemm.cu) against float64."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -139,3 +143,24 @@ def test_sgemm_small_operands_keep_their_bits(M, N, K, ta, tb, exponent):
         b.mul_(scale)
         _check(a, b, ta, tb)
         _check(b.t().contiguous(), a.t().contiguous(), tb, ta)   # the small operand on the right
+
+
+def test_sgemm_as_first_kernel_in_a_capture():
+    """A program may capture before it has run any kernel of the library."""
+    code = """
+import torch
+from tinyinfinitrain_b200._lib import C
+a, b = torch.randn(128, 64, device="cuda"), torch.randn(64, 96, device="cuda")
+out = torch.zeros(128, 96, device="cuda")
+torch.cuda.synchronize()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    C.sgemm(a, b, False, False, out=out)
+graph.replay()
+torch.cuda.synchronize()
+assert (out.double() - a.double() @ b.double()).abs().max().item() < 1e-4
+assert C.status_read(True) == 0
+"""
+    run = subprocess.run([sys.executable, "-c", code], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
+                         capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, run.stderr[-2000:]

@@ -24,8 +24,8 @@ enum TitbError {
 // ---- library status ---------------------------------------------------------
 // One int per device, in device memory, written by kernels whose bounded waits
 // ran out (see common.cuh StatusCode).  titb_status_ptr returns the device
-// pointer (allocating it on first use); titb_status_read copies it to the host
-// after synchronising `stream` and optionally clears it.
+// pointer; titb_status_read copies it to the host after synchronising `stream`
+// and optionally clears it.
 TITB_API int* titb_status_ptr(void);
 TITB_API int titb_status_read(int clear, cudaStream_t stream);
 

@@ -1273,17 +1273,21 @@ static int pick_tile_n(int M, int N, int K, int splits, bool narrow_or_wide = fa
 using namespace titb;
 
 #ifndef TITB_GEMM_PARAM_GATHER
-static int* g_status_dev[64] = {nullptr};
+// One word per device, zero when the library is loaded there: nothing is allocated or cleared at the first launch, which
+// may be inside a graph capture.
+static __device__ int g_status_word;
 
 TITB_API int* titb_status_ptr(void) {
+  static int* address[64] = {nullptr};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) dev = 0;
-  if (!g_status_dev[dev]) {
-    if (cudaMalloc(&g_status_dev[dev], sizeof(int)) != cudaSuccess) return nullptr;
-    cudaMemset(g_status_dev[dev], 0, sizeof(int));
+  if (!address[dev]) {
+    void* p = nullptr;
+    if (cudaGetSymbolAddress(&p, g_status_word) != cudaSuccess) return nullptr;
+    address[dev] = static_cast<int*>(p);
   }
-  return g_status_dev[dev];
+  return address[dev];
 }
 
 TITB_API int titb_status_read(int clear, cudaStream_t stream) {
