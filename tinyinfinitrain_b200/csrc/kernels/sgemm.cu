@@ -16,9 +16,10 @@
 // (without it a value below 2^-110 loses bits), and the sum is scaled back by the first MMA of the product that follows.
 // Values below 2^-125 count to within 2^-148, the two last bits of a subnormal number.  At the upper end bf16(x) is infinite
 // from 2^128 (1 - 2^-9) on, inf - inf appears inside the split of an infinity, and scaled parts or products may overflow where
-// x (from 2^120 on) or the sum (from about 2^114 on) does not.  All of these, and NaN operands, leave a non-finite sum: a warp
-// that finds one computes its 32 x 64 piece of the tile again as a chain of fp32 multiply-adds, which gives IEEE's answer
-// (finfo.min as a mask, infinities) at the pace of the CUDA cores, about a sixth of the usual one.
+// x (from 2^120 on) or the sum (from about 2^114 on) does not.  All of these, and NaN operands, leave a non-finite sum.  A warp
+// that finds one leaves its 32 x 64 piece of the tile out, and when the CTA is through its tiles it computes such pieces again
+// as a chain of fp32 multiply-adds, which gives IEEE's answer (finfo.min as a mask, infinities).  2048 x 3072 x 768 with one
+// infinity: 276 us, with nothing but NaNs: 652 us, against 87 us of finite operands and 480 us of the kernel before.
 //
 // Bound: the six products are 6 x 2 M N K tensor FLOPs, i.e. 278 TFLOP/s of fp32 work at the measured bf16 peak, about four
 // times what 148 SMs x 128 FMA lanes can do.  One CTA works on a 128 x 128 tile:
@@ -37,6 +38,7 @@
 // partial tiles are summed through distributed shared memory in a fixed order -- no workspace, no atomics.
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <limits.h>
 
 #include "api.h"
 #include "ptx_sm100.cuh"
@@ -56,8 +58,9 @@ constexpr float kPartScale = 1 << kPartShift;
 constexpr int kConvWarps = 8, kDrainWarps = 8;
 constexpr int kSThreads = (kConvWarps + kDrainWarps + 1) * 32;
 constexpr int kRedStride = kST + 4;      // floats per row of the partial tile in shared memory (conflict-free 16-byte rows)
-constexpr int kSSmem = kSStages * kSStage + 1024 /*alignment slack*/ + 128 /*barriers*/;
-static_assert(kST * kRedStride * 4 <= kSStages * kSStage, "the partial tile reuses the operand ring");
+constexpr int kSlabK = 16;               // reduction steps that fma_tile stages at a time, behind the partial tile
+constexpr int kSSmem = kSStages * kSStage + 1024 /*alignment slack*/ + 256 /*barriers, pieces left out*/;
+static_assert((kST + 2 * kSlabK) * kRedStride * 4 <= kSStages * kSStage, "the partial tile and the slabs reuse the operand ring");
 
 struct SgemmArgs {
   const float *a, *b;
@@ -118,20 +121,84 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, uint32_t rank) {
   return v;
 }
 
-// acc[j] = sum over k0 <= k < k1 of op(A)[row, k] op(B)[k, col + j], one rounding per step.  The 32 lanes hold different rows and
-// share the columns, so the loads of B are broadcasts.
-__device__ __forceinline__ void fma_chain(float (&acc)[64], const SgemmArgs& p, int row, int col, int k0, int k1) {
-  const long long a_k = p.a_mn ? p.lda : 1, b_k = p.b_mn ? p.ldb : 1, b_n = p.b_mn ? 1 : p.ldb;
-  const float* a = p.a + (p.a_mn ? row : row * p.lda) + k0 * a_k;
-  const float* b = p.b + col * b_n + k0 * b_k;
+// Pieces that the warps which sum the chunks left out: bit n of `tiles` for the CTA's n-th tile, and from tile number `from` on
+// every piece (set by the first one that has no bit).
+struct Redo {
+  uint32_t tiles[kDrainWarps];
+  int from[kDrainWarps];
+  __device__ void clear(int w) {
+    tiles[w] = 0;
+    from[w] = INT_MAX;
+  }
+  __device__ bool any(int w) const { return tiles[w] || from[w] != INT_MAX; }
+  __device__ void leave_out(int w, int tile, int first, int step) {
+    const int n = (tile - first) / step;
+    if (n < 32) tiles[w] |= 1u << n;
+    else from[w] = min(from[w], tile);
+  }
+  __device__ bool left_out(int w, int tile, int first, int step) const {
+    if (!any(w)) return false;
+    const int n = (tile - first) / step;
+    return tile >= from[w] || (n < 32 && (tiles[w] >> n & 1u));
+  }
+};
+
+// Computes one tile over k0 <= k < k1 on the CUDA cores, one rounding per step in ascending order, and hands the values of the
+// pieces in the mask `pieces` to put(row, column, value).  The whole CTA calls it; 512 threads hold 8 x 4 values each.  It comes
+// after the tile loop so that its registers are not the tile loop's: in the loop, it made every call 8 % slower.
+template <typename Put>
+__device__ __forceinline__ void fma_tile(const SgemmArgs& p, int m0, int n0, int k0, int k1, uint32_t pieces, float* slab, Put put) {
+  float* as = slab;
+  float* bs = slab + kSlabK * kRedStride;
+  const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
+  const bool work = tid < 512;
+  float acc[8][4];
 #pragma unroll
-  for (int j = 0; j < 64; ++j) acc[j] = 0.f;
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+  // element e of a slab: neighbouring threads read along the contiguous direction of the operand
+  auto fill = [&](float* dst, const float* base, long long ld, int mn, int r0, int rows, int k) {
+#pragma unroll
+    for (int i = 0; i < kSlabK * kST / 512; ++i) {
+      const int e = i * 512 + tid;
+      const int s = mn ? e / kST : e % kSlabK, r = mn ? e % kST : e / kSlabK;
+      const bool in = k + s < k1 && r0 + r < rows;
+      dst[s * kRedStride + r] = in ? __ldg(base + (mn ? (k + s) * ld + r0 + r : (r0 + r) * ld + k + s)) : 0.f;
+    }
+  };
 #pragma unroll 1
-  for (int k = k0; k < k1; ++k, a += a_k, b += b_k) {
-    const float x = __ldg(a);
+  for (int k = k0; k < k1; k += kSlabK) {
+    __syncthreads();   // the slabs before have been read
+    if (work) {
+      fill(as, p.a, p.lda, p.a_mn, m0, p.M, k);
+      fill(bs, p.b, p.ldb, p.b_mn, n0, p.N, k);
+    }
+    __syncthreads();
+    if (work) {
+#pragma unroll 1
+      for (int s = 0; s < kSlabK; ++s) {
+        float x[8], y[4];
 #pragma unroll
-    for (int j = 0; j < 64; ++j)
-      if (col + j < p.N) acc[j] = fmaf(x, __ldg(b + j * b_n), acc[j]);
+        for (int h = 0; h < 2; ++h)
+          *reinterpret_cast<float4*>(x + 4 * h) = *reinterpret_cast<const float4*>(as + s * kRedStride + h * 64 + ty * 4);
+        *reinterpret_cast<float4*>(y) = *reinterpret_cast<const float4*>(bs + s * kRedStride + tx * 4);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(x[i], y[j], acc[i][j]);
+      }
+    }
+  }
+  if (!work) return;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = (i >> 2) * 64 + ty * 4 + (i & 3);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int c = tx * 4 + j;
+      if (pieces >> ((c >> 6) * 4 + (r >> 5)) & 1u) put(r, c, acc[i][j]);
+    }
   }
 }
 
@@ -144,6 +211,7 @@ __global__ void __launch_bounds__(kSThreads, 1) sgemm_split3_kernel(const SgemmA
   uint64_t* acc_empty = acc_full + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile uint32_t* abort_flag = tmem_slot + 1;
+  Redo* redo = reinterpret_cast<Redo*>(smem + kSStages * kSStage + 128);
   const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -156,6 +224,7 @@ __global__ void __launch_bounds__(kSThreads, 1) sgemm_split3_kernel(const SgemmA
       ptx::mbar_init(&acc_empty[b], kDrainWarps);
     }
     *abort_flag = 0;
+    for (int w = 0; w < kDrainWarps; ++w) redo->clear(w);
     ptx::mbar_fence_init();
   }
   if (warp == kConvWarps + kDrainWarps) {
@@ -293,8 +362,10 @@ __global__ void __launch_bounds__(kSThreads, 1) sgemm_split3_kernel(const SgemmA
       float finite = 0.f;
 #pragma unroll
       for (int j = 0; j < 64; ++j) finite = fmaf(acc[j], 0.f, finite);
-      if (gc < p.N && __any_sync(0xffffffffu, !(finite == 0.f)))
-        fma_chain(acc, p, min(gr, p.M - 1), gc, c0 * kSK, min(p.K, c1 * kSK));
+      // (kept in shared memory: in registers this made the whole kernel spill)
+      if (gc < p.N && __any_sync(0xffffffffu, !(finite == 0.f)) && lane == 0) redo->leave_out(warp - kConvWarps, tile, first, step);
+      __syncwarp();
+      if (redo->left_out(warp - kConvWarps, tile, first, step)) continue;   // a cluster works on one tile: ends its loop
       if (p.split > 1) {
         // every MMA of this CTA has finished (the last accumulator was read), so the operand ring is free
         float* red = reinterpret_cast<float*>(smem) + row * kRedStride + half * 64;
@@ -330,6 +401,25 @@ __global__ void __launch_bounds__(kSThreads, 1) sgemm_split3_kernel(const SgemmA
   ptx::tc_fence_before_sync();
   __syncwarp();   // the lanes of the MMA warp meet again
   __syncthreads();
+  bool again = false;
+  for (int w = 0; w < kDrainWarps; ++w) again |= redo->any(w);
+  if (again && !*abort_flag) {
+    float* red = reinterpret_cast<float*>(smem);
+    for (int tile = first; tile < tiles; tile += step) {
+      uint32_t pieces = 0;
+      for (int w = 0; w < kDrainWarps; ++w) pieces |= static_cast<uint32_t>(redo->left_out(w, tile, first, step)) << w;
+      if (!pieces) continue;
+      const int m0 = (tile % tiles_m) * kST, n0 = (tile / tiles_m) * kST;
+      fma_tile(p, m0, n0, c0 * kSK, min(p.K, c1 * kSK), pieces, red + kST * kRedStride, [&](int r, int c, float v) {
+        if (p.split > 1) {
+          red[r * kRedStride + c] = v;
+        } else if (m0 + r < p.M && n0 + c < p.N) {
+          float* out = p.c + static_cast<long long>(m0 + r) * p.N + n0 + c;
+          *out = p.accumulate ? *out + v : v;
+        }
+      });
+    }
+  }
   if (p.split > 1) {
     ptx::cluster_sync_all();   // every CTA's partial tile is in its shared memory
     const int rows = kST / p.split, tile = first;
