@@ -27,6 +27,22 @@ def _status_ok():
 
 
 @pytest.mark.parametrize("B,T,Hq,Hkv,hd", [(3, 1, 2, 2, 64), (2, 127, 2, 1, 128), (2, 129, 4, 2, 128), (3, 257, 2, 1, 64)])
+def test_attention_forward_tiles_end_with_their_sequence(B, T, Hq, Hkv, hd):
+    """NaNs and infinities in the other sequences leave the output and the row statistics of sequence 0 as they were, to the
+    bit: rows past its end read as zero instead of meeting probabilities of zero."""
+    torch.manual_seed(24)
+    q = torch.randn(B, T, Hq, hd, device=DEV).to(BF)
+    k, v = (torch.randn(B, T, Hkv, hd, device=DEV).to(BF) for _ in range(2))
+    o, lse = (t.clone() for t in C.attn_fwd(q, k, v, hd ** -0.5))
+    for bad in (float("nan"), float("inf")):
+        for t in (q, k, v):
+            t[1:] = bad
+        o2, lse2 = C.attn_fwd(q, k, v, hd ** -0.5)
+        _status_ok()
+        assert torch.equal(o2[0], o[0]) and torch.equal(lse2[0], lse[0])
+
+
+@pytest.mark.parametrize("B,T,Hq,Hkv,hd", [(3, 1, 2, 2, 64), (2, 127, 2, 1, 128), (2, 129, 4, 2, 128), (3, 257, 2, 1, 64)])
 def test_attention_backward_tiles_end_with_their_sequence(B, T, Hq, Hkv, hd):
     """The last tile of a sequence reads zeros past its end and adds nothing there: NaNs in the other sequences leave the
     gradients of sequence 0 as they were (dK and dV to the bit; dQ is a sum of at most three partials in any order, each

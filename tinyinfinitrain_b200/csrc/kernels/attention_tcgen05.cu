@@ -34,8 +34,6 @@
 
 namespace titb {
 
-bool make_tmap_bf16_2d(CUtensorMap* m, const void* base, uint64_t inner, uint64_t outer, uint64_t ld,
-                       uint32_t box_inner, uint32_t box_outer);
 bool make_tmap_tokens(CUtensorMap* m, const void* base, int fp32, uint64_t width, uint64_t T, uint64_t B, uint64_t ld,
                       uint32_t box_width, uint32_t box_tokens);
 
@@ -173,21 +171,21 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
       ptx::mbar_expect_tx(q_full, Cfg::kTileBytes);
 #pragma unroll
       for (int c = 0; c < HD / 64; ++c)
-        ptx::tma_load_2d(smem + Cfg::kQ + c * kChunkBytes, &tq, q_full, h * HD + c * 64, b * p.T + q0);
+        ptx::tma_load_3d(smem + Cfg::kQ + c * kChunkBytes, &tq, q_full, h * HD + c * 64, q0, b);
       for (int j = 0; j < nblk; ++j) {
         const int st = j & 1;
         if (!ptx::mbar_wait(&k_empty[st], ((j >> 1) & 1) ^ 1u, abort_flag)) break;
         ptx::mbar_expect_tx(&k_full[st], Cfg::kTileBytes);
 #pragma unroll
         for (int c = 0; c < HD / 64; ++c)
-          ptx::tma_load_2d(smem + Cfg::kK + st * Cfg::kTileBytes + c * kChunkBytes, &tk, &k_full[st],
-                           hk * HD + c * 64, b * p.T + j * kBlk);
+          ptx::tma_load_3d(smem + Cfg::kK + st * Cfg::kTileBytes + c * kChunkBytes, &tk, &k_full[st], hk * HD + c * 64,
+                           j * kBlk, b);
         if (!ptx::mbar_wait(&v_empty[st], ((j >> 1) & 1) ^ 1u, abort_flag)) break;
         ptx::mbar_expect_tx(&v_full[st], Cfg::kTileBytes);
 #pragma unroll
         for (int c = 0; c < HD / 64; ++c)
-          ptx::tma_load_2d(smem + Cfg::kV + st * Cfg::kTileBytes + c * kChunkBytes, &tv, &v_full[st],
-                           hk * HD + c * 64, b * p.T + j * kBlk);
+          ptx::tma_load_3d(smem + Cfg::kV + st * Cfg::kTileBytes + c * kChunkBytes, &tv, &v_full[st], hk * HD + c * 64,
+                           j * kBlk, b);
       }
     }
   } else if (warp == 1) {
@@ -871,11 +869,12 @@ static int attn_fwd_launch(const TitbAttnDesc* d, cudaStream_t st) {
     if (e != cudaSuccess) return static_cast<int>(e);
     attr_set[dev] = true;
   }
-  const uint64_t rows = static_cast<uint64_t>(d->B) * d->T;
+  // the maps end with a sequence: rows of the next one would meet probabilities of zero, which do not stop a NaN
+  const uint64_t B = d->B, T = d->T, wq = static_cast<uint64_t>(d->Hq) * HD, wkv = static_cast<uint64_t>(d->Hkv) * HD;
   CUtensorMap tq, tk, tv;
-  if (!make_tmap_bf16_2d(&tq, d->q, static_cast<uint64_t>(d->Hq) * HD, rows, d->q_stride_t, 64, kBlk) ||
-      !make_tmap_bf16_2d(&tk, d->k, static_cast<uint64_t>(d->Hkv) * HD, rows, d->k_stride_t, 64, kBlk) ||
-      !make_tmap_bf16_2d(&tv, d->v, static_cast<uint64_t>(d->Hkv) * HD, rows, d->v_stride_t, 64, kBlk))
+  if (!make_tmap_tokens(&tq, d->q, 0, wq, T, B, d->q_stride_t, 64, kBlk) ||
+      !make_tmap_tokens(&tk, d->k, 0, wkv, T, B, d->k_stride_t, 64, kBlk) ||
+      !make_tmap_tokens(&tv, d->v, 0, wkv, T, B, d->v_stride_t, 64, kBlk))
     return TITB_ERR_TENSOR_MAP;
   AttnArgs a{};
   a.B = d->B; a.T = d->T; a.Hq = d->Hq; a.Hkv = d->Hkv; a.hd = HD;
