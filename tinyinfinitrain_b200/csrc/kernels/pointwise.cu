@@ -385,6 +385,7 @@ TITB_API int titb_rope_strided(const void* x, void* y, int B, int T, int H, int 
   const int vn = dtype == 1 ? 8 : 4;
   if ((hd / 2) % vn) return (int)cudaErrorInvalidValue;
   const int hv = hd / 2 / vn;
+  if (H <= 0 || hv <= 0) return 0;
   // as many heads per thread as leave every SM 512 threads, 8 at most
   long long per = BT * H * hv / (device_sm_count() * 512LL);
   per = per < 1 ? 1 : per > 8 ? 8 : per;
