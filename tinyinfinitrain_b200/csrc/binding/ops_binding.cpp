@@ -95,7 +95,9 @@ std::vector<Tensor> gemm(const Tensor& a, const Tensor& b, bool a_mn, bool b_mn,
     TORCH_CHECK(alpha->is_cuda() && alpha->scalar_type() == at::kFloat && alpha->numel() == 1, "titb200 gemm: alpha must be a CUDA fp32 scalar");
     d.alpha = alpha->data_ptr();
   }
-  int s = splits > 0 ? (int)splits : titb_gemm_pick_splits((int)M, (int)N, (int)K, !titb_gemm_split_in_place(&d));
+  int s = splits > 0                       ? (int)splits
+          : titb_gemm_split_in_place(&d) ? titb_gemm_pick_splits((int)M, (int)N, (int)K)
+                                         : titb_gemm_pick_splits_workspace((int)M, (int)N, (int)K);
   if (epilogue != TITB_EPI_NONE || (N & 3)) s = 1;
   // bf16 outputs go through an fp32 workspace and a reduction kernel: worth it only for very long reductions
   // (the vocabulary projection's input gradient, K = 50304)

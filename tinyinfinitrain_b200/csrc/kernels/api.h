@@ -92,9 +92,10 @@ TITB_API int titb_gemm_bf16(const TitbGemmDesc* d, cudaStream_t stream);
 // as mapped on this GPU (for r == rank it may alias the local copy: then nothing is moved), `coll->flags` N / 128
 // uint32 words of scratch.  The caller orders the launch after the owners' last writes (device barrier).
 TITB_API int titb_gemm_param_gather_bf16(const TitbGemmDesc* d, cudaStream_t stream);
-// Picks the split-K factor the heuristic would use (so callers can size the workspace).
-// workspace: 1 when the partial tiles go through the workspace and a second kernel, 0 when they meet in the output.
-TITB_API int titb_gemm_pick_splits(int M, int N, int K, int workspace);
+// Picks the split-K factor the heuristic would use (so callers can size the workspace): for partial tiles that meet in the
+// output, and for partial tiles that go through the workspace and a second kernel (see titb_gemm_split_in_place).
+TITB_API int titb_gemm_pick_splits(int M, int N, int K);
+TITB_API int titb_gemm_pick_splits_workspace(int M, int N, int K);
 // Tile width (128, 192 or 256) the GEMM takes for this shape and split-K factor when the descriptor leaves tile_n 0.
 TITB_API int titb_gemm_pick_tile(int M, int N, int K, int splits);
 // 1 when a split-K call with this descriptor sums its partial tiles in the output itself (fp32 output, no fused

@@ -1304,7 +1304,7 @@ TITB_API void titb_gemm_set_tma_store(int enabled) { g_no_tma_store = enabled ? 
 
 TITB_API int titb_gemm_pick_tile(int M, int N, int K, int splits) { return pick_tile_n(M, N, K, splits < 1 ? 1 : splits); }
 
-TITB_API int titb_gemm_pick_splits(int M, int N, int K, int workspace) {
+static int pick_splits(int M, int N, int K, bool workspace) {
   // Joint choice of split-K factor and tile width by estimated duration (plan_cost): the reduction is split when the
   // output has too few tiles to fill the GPU -- weight gradients: small outputs, K = the token count -- and each
   // split still runs a pipeline of at least 8 k-blocks.  (Callers use the result only where the partial tiles can
@@ -1317,12 +1317,15 @@ TITB_API int titb_gemm_pick_splits(int M, int N, int K, int workspace) {
     if (s > 1 && kb / s < 8) break;
     for (int bn : {256, 192, 128}) {
       if (bn > 128 && N <= 128) continue;
-      const double c = plan_cost(M, N, K, bn, s, sms, workspace != 0);
+      const double c = plan_cost(M, N, K, bn, s, sms, workspace);
       if (c < best) { best = c; best_s = s; }
     }
   }
   return best_s;
 }
+
+TITB_API int titb_gemm_pick_splits(int M, int N, int K) { return pick_splits(M, N, K, false); }
+TITB_API int titb_gemm_pick_splits_workspace(int M, int N, int K) { return pick_splits(M, N, K, true); }
 #endif  // !TITB_GEMM_PARAM_GATHER
 
 static bool deterministic_reductions() {
