@@ -30,9 +30,9 @@
 // Splitting in the kernel costs about 1000 issue slots per chunk and scheduler, under the 1536 cycles of its MMAs; a
 // separate split pass would write and read another 6 bytes per element.
 // Measured (B200, GPT-2 124M layers, forward / input gradient / weight gradient), before = a 64 x 64 CUDA-core kernel:
-//   2048 tokens, 3072 x 768:  473 / 669 / 698 us before,  85 / 102 / 72 us now (114 / 95 / 134 TFLOP/s)
-//   2048 tokens, 50304 x 768: 7.1 / 11.6 / 10.6 ms before, 1.11 / 1.60 / 1.09 ms now
-//   128 tokens,  50304 x 768: 511 / 8908 / 685 us before,  91 / 218 / 102 us now
+//   2048 tokens, 3072 x 768:  473 / 669 / 698 us before,  86 / 105 / 76 us now (112 / 92 / 127 TFLOP/s)
+//   2048 tokens, 50304 x 768: 7.1 / 11.6 / 10.6 ms before, 1.06 / 1.53 / 1.11 ms now
+//   128 tokens,  50304 x 768: 511 / 8908 / 685 us before,  92 / 213 / 102 us now
 //   rms error against float64 at K = 768: 5.0e-7 before, 1.0e-7 now; at K = 50304: 4.0e-6 before, 2e-7 to 5e-7 now
 // Few output tiles (small batches, long reductions): a cluster of 2, 4 or 8 CTAs shares one tile's reduction, and the
 // partial tiles are summed through distributed shared memory in a fixed order -- no workspace, no atomics.
@@ -457,7 +457,9 @@ __global__ void __launch_bounds__(kSThreads, 1) sgemm_split3_kernel(const SgemmA
 }
 
 // CTAs per tile: the fewest rounds of chunks on the busiest SM, with a charge for the exchange of the partial tiles (about
-// three chunks).  A part keeps at least one chunk.
+// three chunks).  Parts are whole multiples of ceil(chunks / parts): the last ones may have nothing to add but zeros (nine
+// chunks over eight parts), which costs nothing, as the others take no longer for it.  That all clusters run at the same time
+// is assumed, not asked: clusters of eight may wait for room within a group of SMs.
 int pick_split(int tiles, int nchunk, int sms) {
   int best = 1;
   double cost = 1e30;

@@ -110,7 +110,7 @@ def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("kernel", choices=["gemm", "gemm_nt", "gemm_wgrad", "attn_fwd", "attn_bwd", "layernorm_fwd", "layernorm_bwd",
                                        "xent", "adam", "gelu_gemm", "ag_gemm", "gemm_rs", "rs_adam", "clip", "embedding_bwd",
-                                       "reduce", "transpose_view", "colsum", "param_gather_gemm", "gemm_sweep"])
+                                       "reduce", "transpose_view", "colsum", "param_gather_gemm", "gemm_sweep", "sgemm"])
     ap.add_argument("--model", default="gpt2", choices=["gpt2", "gpt2xl", "llama1b"], help="gemm_sweep: whose layer shapes")
     ap.add_argument("--deterministic", action="store_true", help="embedding_bwd: sorted segment reduction instead of atomics")
     ap.add_argument("--world", type=int, default=4)
@@ -153,6 +153,11 @@ def main():
             A, B = torch.randn(K, M, device=dev).to(bf), torch.randn(K, N, device=dev).to(bf)
             out = torch.zeros(M, N, device=dev)
             fn = lambda: C.gemm(A, B, True, True, out=out, accumulate=True, tile_n=a.tile_n)
+    elif a.kernel == "sgemm":          # fp32 operands, forward layout; six bf16 products per fp32 product
+        A, B = torch.randn(a.m, a.k, device=dev), torch.randn(a.n, a.k, device=dev)
+        flops = 2.0 * a.m * a.n * a.k
+        bytes_ = 4.0 * (a.m * a.k + a.n * a.k + a.m * a.n)
+        fn = lambda: C.sgemm(A, B, False, True)
     elif a.kernel in ("attn_fwd", "attn_bwd"):
         Hkv = a.hkv or a.h
         W = (a.h + 2 * Hkv) * a.hd
