@@ -513,6 +513,26 @@ def test_parameter_gather_gemm_on_one_gpu(world, npr, M, K, bias):
     _status_ok()
 
 
+@pytest.mark.parametrize("world,npr,M,K", [(1, 256, 300, 128), (2, 1024, 2048, 256), (4, 1024, 4096, 320)])
+def test_parameter_gather_gemm_with_residual_on_one_gpu(world, npr, M, K):
+    """The residual comes a tile ahead of the accumulator.  CTAs that copy sit out the first rounds of the tile list and the
+    others share them, so the order of a CTA's tiles is not a plain stride: fewer tiles than CTAs, and several rounds."""
+    torch.manual_seed(30)
+    N = npr * world
+    Wt = (torch.randn(N, K, device=DEV) * 0.2).to(BF)
+    x, res = torch.randn(M, K, device=DEV).to(BF), (4 * torch.randn(M, N, device=DEV)).to(BF)
+    b = torch.randn(N, device=DEV).to(BF)
+    ref = x.float() @ Wt.float().t() + b.float() + res.float()
+    copies = [torch.full((N, K), float("nan"), device=DEV, dtype=BF) for _ in range(world)]
+    for r in range(world):
+        copies[r][r * npr:(r + 1) * npr] = Wt[r * npr:(r + 1) * npr]
+    ptrs = [copies[r].data_ptr() + r * npr * K * 2 for r in range(world)]
+    y = C.gemm_param_gather(x, copies[0], ptrs, 0, epilogue=ops.EPI_BIAS_RESIDUAL, bias=b, aux_in=res)[0]
+    _status_ok()
+    # one rounding of the result to bf16, and the fp32 sum in another order
+    assert bool(((y.float() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-4).all())
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, BF])
 @pytest.mark.parametrize("V,vocab,shards", [(512, 500, 2), (1024, 1000, 4), (96, 50, 3)])
 def test_vocab_parallel_xent_kernels_match_full_softmax(dtype, V, vocab, shards):

@@ -1017,16 +1017,15 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
       // Residual / pre-activation tiles are fetched one chunk ahead by TMA into the warp's aux staging tile.
       constexpr int kChunksPerTile = BN / 64;
       uint64_t* my_aux_bar = &aux_bar[warp - 2];
-      const int my_tiles = cta < num_tiles ? (num_tiles - cta + ncta - 1) / ncta : 0;
-      const int total_chunks = my_tiles * kChunksPerTile;
-      auto issue_aux_load = [&](int g) {  // g: running chunk index over this CTA's tiles
-        const int t_local = g / kChunksPerTile;
-        const TileCoord t2 = tile_coord(p, cta + t_local * ncta, tiles_m, tiles_n, BN, kTileM, row_off);
+      auto issue_aux_load = [&](int g) {  // g: running chunk index over this CTA's tiles, in the order in which it takes them
+        const int t = walk.tile(walk.first_round() + g / kChunksPerTile);
+        if (t >= num_tiles || !ptx::elect_one()) return;
+        const TileCoord t2 = tile_coord(p, t, tiles_m, tiles_n, BN, kTileM, row_off);
         ptx::mbar_expect_tx(my_aux_bar, 4096);
         ptx::tma_load_2d(wo.aux, &tma_aux, my_aux_bar, t2.n0 + (g % kChunksPerTile) * 64, t2.m0 + quad * 32);
       };
       int gchunk = 0;
-      if (p.aux_tma_load && total_chunks > 0 && ptx::elect_one()) issue_aux_load(0);
+      if (p.aux_tma_load) issue_aux_load(0);
       for (int rnd = walk.first_round(), tile; (tile = walk.tile(rnd)) < num_tiles; ++rnd, ++it) {
         const TileCoord tc = tile_coord(p, tile, tiles_m, tiles_n, BN, kTileM, row_off);
         const int m0 = tc.m0, n0 = tc.n0;
@@ -1050,8 +1049,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
                 aux_row[u] = *reinterpret_cast<const uint4*>(wo.aux + lane * 128 + ((u ^ (lane & 7)) << 4));
             }
             __syncwarp();
-            ++gchunk;
-            if (gchunk < total_chunks && ptx::elect_one()) issue_aux_load(gchunk);
+            issue_aux_load(++gchunk);
           }
           uint32_t r0[32], r1[32];
           if (col0 < p.N) {
@@ -1234,6 +1232,7 @@ static int g_no_tma_store = 0;  // set by titb_gemm_set_tma_store(0): A/B switch
 // shapes of GPT-2 124M / XL and LLaMA-3 1B / 8B layers at 256 to 8192 tokens (forward, input and weight gradients, each
 // timed with every width and split): the choices are 0.4 % off the fastest configuration on average, where constants from
 // before MMAs were issued by an elected lane, when every width took the same time per k-block, were 9.7 % off.
+// The fused collectives take their tile width from it too, without having been part of the fit.
 //   k-block   how long 64 reduction steps of a tile take: the MMAs, or on a full machine the operand bytes out of L2
 //   fixed     launch, pipeline fill, the last epilogue
 //   epilogue  what the next main loop does not hide of an epilogue
