@@ -13,11 +13,12 @@
 namespace titb {
 
 // Bound: memory, 16 bytes read and 14 (bf16 weights) written per parameter.  A CTA updates kAdamPerCta consecutive parameters
-// and ends: 8 per thread, all 8 loads of a thread in flight before the first use, and the five streams of the CTAs that run
+// and ends: 4 per thread, the four loads of a thread in flight before the first use, and the five streams of the CTAs that run
 // at the same time lie close together (a grid-wide stride spread each stream over the whole buffer).  The state is touched
 // once a step and passes through the caches as streaming data; the weights that the next forward pass reads stay.
-// Measured (B200, bf16 weights): 124 M parameters 631 -> 575 us, 1.5 G 7576 -> 6784 us (6.63 TB/s).
-constexpr int kAdamVecs = 2;
+// Measured (B200, bf16 weights; grid-wide stride -> now): 100 K parameters 2.5 -> 2.2 us, 2 M 7.1 -> 7.1 us, 124 M 631 -> 565 us,
+// 780 M 3.97 -> 3.53 ms.  Two vectors per thread and half the CTAs: 2.9 us, 7.5 us, 566 us, 3.54 ms.
+constexpr int kAdamVecs = 1;
 constexpr int kAdamPerCta = 256 * 4 * kAdamVecs;
 
 template <typename LP>
