@@ -54,6 +54,22 @@ def test_sgemm_is_as_accurate_as_an_fp32_chain(M, N, K, positive):
     assert err <= (chain.double() - ref).norm()
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 1, 2), (63, 65, 15), (64, 64, 16), (65, 200, 17), (64, 64, 31), (1, 5000, 32), (300, 70, 33),
+                                   (2048, 2048, 32), (2048, 2050, 32), (2049, 2500, 16), (2047, 2049, 33)])
+@pytest.mark.parametrize("ta,tb", [(False, False), (False, True), (True, False), (True, True)])
+def test_sgemm_of_short_reductions(M, N, K, ta, tb):
+    """Both sides of the lines between the CUDA-core kernels (a rounding per step) and the tensor-core one."""
+    a, b, A, B = _operands(M, N, K, ta, tb, 8)
+    ref, mag = A.double() @ B.double(), A.double().abs() @ B.double().abs()
+    bound = (max(K, 2 * 5 + 1) + 2) * 2.0 ** -24 * mag
+    out = C.sgemm(a, b, ta, tb)
+    assert bool(((out.double() - ref).abs() <= bound).all())
+    acc = torch.ones_like(out)
+    C.sgemm(a, b, ta, tb, out=acc, accumulate=True)
+    assert torch.equal(acc, out + 1)
+    assert C.status_read(True) == 0
+
+
 def test_sgemm_exact_on_small_integers_and_repeatable():
     g = torch.Generator(device=DEV).manual_seed(2)
     a = torch.randint(-64, 65, (200, 300), device=DEV, generator=g).float()
@@ -148,7 +164,7 @@ def test_sgemm_small_operands_keep_their_bits(M, N, K, ta, tb, exponent):
 def test_sgemm_non_finite_operands_in_late_tiles():
     """More tiles per CTA (33) than the mask of left-out pieces has bits."""
     M = N = 69 * 128
-    a, b, A, B = _operands(M, N, 3, False, True, 7)
+    a, b, A, B = _operands(M, N, 33, False, True, 7)
     A[5, 1] = INF
     A[68 * 128 + 5, 1] = -INF
     A[68 * 128 + 70, 0] = NAN

@@ -35,7 +35,8 @@
 //   128 tokens,  50304 x 768: 511 / 8908 / 685 us before,  92 / 213 / 102 us now
 //   rms error against float64 at K = 768: 5.0e-7 before, 1.0e-7 now; at K = 50304: 4.0e-6 before, 2e-7 to 5e-7 now
 // Few output tiles (small batches, long reductions): a cluster of 2, 4 or 8 CTAs shares one tile's reduction, and the
-// partial tiles are summed through distributed shared memory in a fixed order -- no workspace, no atomics.
+// partial tiles are summed through distributed shared memory in a fixed order -- no workspace, no atomics.  Very short
+// reductions: sgemm_short_kernel.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <limits.h>
@@ -456,6 +457,79 @@ __global__ void __launch_bounds__(kSThreads, 1) sgemm_split3_kernel(const SgemmA
   if (threadIdx.x == 0 && *abort_flag) atomicExch(p.status, kStatusMbarTimeout);
 }
 
+// Reductions of at most KM steps: a 64 x 64 tile per CTA on the CUDA cores, the whole reduction loaded at once, 4 x 4 values per
+// thread, one rounding per step in ascending order.  A chunk of the kernel above is 64 steps deep, and its set-up (barriers,
+// tensor memory, two hand-overs between warps) takes longer than such a product.  Measured (B200, us, K = 16 / 32, the kernel
+// above -> this one): 16 x 16 7.1 -> 2.1 / 7.1 -> 3.1, 1024 x 1024 8.1 -> 3.2 / 8.1 -> 4.8, 2048 x 2048 12.8 -> 7.2 / 12.9 -> 12.2,
+// 4096 x 4096 34.6 -> 24.3 / 34.8 -> 42.0.
+template <int KM>
+__global__ void __launch_bounds__(256) sgemm_short_kernel(const SgemmArgs p) {
+  dependency_wait();
+  dependents_launch();
+  __shared__ float4 as[KM][17], bs[KM][17];
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int tiles_m = (p.M + 63) / 64;
+  const int m0 = static_cast<int>(blockIdx.x % tiles_m) * 64, n0 = static_cast<int>(blockIdx.x / tiles_m) * 64;
+  float va[KM / 4], vb[KM / 4];
+  // neighbouring threads read along the contiguous direction of the operand
+  auto at = [&](int i, int mn, int& k, int& r) {
+    const int e = i * 256 + tid;
+    k = mn ? e >> 6 : e % KM;
+    r = mn ? e & 63 : e / KM;
+  };
+  auto load = [&](float (&v)[KM / 4], const float* base, long long ld, int mn, int r0, int rows) {
+#pragma unroll
+    for (int i = 0; i < KM / 4; ++i) {
+      int k, r;
+      at(i, mn, k, r);
+      v[i] = k < p.K && r0 + r < rows ? __ldg(base + (mn ? k * ld + r0 + r : (r0 + r) * ld + k)) : 0.f;
+    }
+  };
+  auto store = [&](const float (&v)[KM / 4], float4 (&dst)[KM][17], int mn) {
+#pragma unroll
+    for (int i = 0; i < KM / 4; ++i) {
+      int k, r;
+      at(i, mn, k, r);
+      reinterpret_cast<float*>(dst[k])[r] = v[i];
+    }
+  };
+  load(va, p.a, p.lda, p.a_mn, m0, p.M);
+  load(vb, p.b, p.ldb, p.b_mn, n0, p.N);
+  store(va, as, p.a_mn);
+  store(vb, bs, p.b_mn);
+  __syncthreads();
+  float acc[4][4] = {};
+#pragma unroll 8
+  for (int k = 0; k < p.K; ++k) {
+    const float4 x = as[k][ty], y = bs[k][tx];
+    const float xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(xs[i], ys[j], acc[i][j]);
+  }
+  const int c = n0 + tx * 4;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = m0 + ty * 4 + i;
+    if (r >= p.M) break;
+    float* out = p.c + static_cast<long long>(r) * p.N + c;
+    if (p.c_vec && c + 4 <= p.N) {
+      float4* o = reinterpret_cast<float4*>(out);
+      float4 v = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+      if (p.accumulate) {
+        const float4 old = *o;
+        v.x += old.x; v.y += old.y; v.z += old.z; v.w += old.w;
+      }
+      *o = v;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (c + j < p.N) out[j] = p.accumulate ? out[j] + acc[i][j] : acc[i][j];
+    }
+  }
+}
+
 // CTAs per tile: the fewest rounds of chunks on the busiest SM, with a charge for the exchange of the partial tiles (about
 // three chunks).  Parts are whole multiples of ceil(chunks / parts): the last ones may have nothing to add but zeros (nine
 // chunks over eight parts), which costs nothing, as the others take no longer for it.  That all clusters run at the same time
@@ -483,6 +557,22 @@ TITB_API int titb_sgemm(const float* A, const float* B, float* C, int M, int N, 
   (void)cudaGetLastError();
   if (K <= 0)
     return accumulate ? 0 : static_cast<int>(cudaMemsetAsync(C, 0, sizeof(float) * static_cast<size_t>(M) * N, stream));
+  auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  SgemmArgs a{};
+  a.a = A; a.b = B; a.c = C;
+  a.M = M; a.N = N; a.K = K;
+  a.a_mn = trans_a ? 1 : 0;
+  a.b_mn = trans_b ? 0 : 1;      // op(B) = B^T means B is stored [N, K]
+  a.lda = trans_a ? M : K;
+  a.ldb = trans_b ? K : N;
+  a.accumulate = accumulate;
+  a.c_vec = (reinterpret_cast<uintptr_t>(C) & 31) == 0 && !(N & 7);
+  // where the lines lie: see sgemm_short_kernel
+  if (K <= 16 || (K <= 32 && static_cast<long long>(M) * N <= 1 << 22)) {
+    const cudaError_t e = launch_dependent(K <= 16 ? sgemm_short_kernel<16> : sgemm_short_kernel<32>,
+                                           static_cast<unsigned>(((M + 63) / 64) * ((N + 63) / 64)), 256, 0, stream, a);
+    return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
+  }
   static bool attr_set[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -492,18 +582,8 @@ TITB_API int titb_sgemm(const float* A, const float* B, float* C, int M, int N, 
     if (e != cudaSuccess) return static_cast<int>(e);
     attr_set[dev] = true;
   }
-  auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
-  SgemmArgs a{};
-  a.a = A; a.b = B; a.c = C;
-  a.M = M; a.N = N; a.K = K;
-  a.a_mn = trans_a ? 1 : 0;
-  a.b_mn = trans_b ? 0 : 1;      // op(B) = B^T means B is stored [N, K]
-  a.lda = trans_a ? M : K;
-  a.ldb = trans_b ? K : N;
   a.a_vec = al16(A) && !(a.lda & 3);
   a.b_vec = al16(B) && !(a.ldb & 3);
-  a.c_vec = (reinterpret_cast<uintptr_t>(C) & 31) == 0 && !(N & 7);
-  a.accumulate = accumulate;
   a.status = titb_status_ptr();
   if (!a.status) return static_cast<int>(cudaErrorMemoryAllocation);
   const int sms = device_sm_count();
